@@ -55,6 +55,13 @@ def _log(rng, lo, hi):
     return int(round(math.exp(rng.uniform(math.log(lo), math.log(hi)))))
 
 
+def _smooth(n):
+    for p in (2, 3, 5, 7, 11, 13):
+        while n % p == 0:
+            n //= p
+    return n == 1
+
+
 def draw(rng):
     kind = rng.choice(["apply"] * 6 + ["gram"] * 2 + ["update"] * 2 + ["solve", "host"])
     if kind in ("apply", "host"):
@@ -64,8 +71,8 @@ def draw(rng):
         elif style == "smooth":
             n = [rng.choice([16, 20, 24, 30, 32, 36, 40, 45, 48, 50, 54, 60, 64, 72, 80, 90, 96, 100, 108, 120, 128])
                  for _ in range(3)]
-        else:
-            n = [_log(rng, 16, 80) for _ in range(3)]
+        else:  # any length the library takes: no prime factor above 13
+            n = [rng.choice([k for k in range(16, 81) if _smooth(k)]) for _ in range(3)]
         size = n[0] * n[1] * n[2]
         op = rng.choice(["lrep", "lrep", "tlrep", "m", "k"])
         if kind == "host":
