@@ -54,6 +54,8 @@ struct bdgd_ctx {
   double2 *d_roots64[3];
   float2 *d_roots32[3];
   double *d_kx2[3];
+  double2 *h_roots64[3];  // host copies of the roots
+  float2 *h_roots32[3];
   // physics (FP64 and FP32 copies)
   double *ltK64, *ltM64, *pK64, *pM64;
   float *ltK32, *ltM32, *pK32, *pM32;
@@ -77,6 +79,7 @@ struct bdgd_ctx {
   // FFT pass family per (operator, precision) chosen by the autotuner:
   // 0 not tuned, 1 register lines, 2 compile-time shared-memory stages
   signed char tune[16][2];
+  signed char tune_lines[16][2];  // the register family runs as line passes
   float tune_ms[16][2][2];
   int force_path;   // set while the autotuner times one family
   // CUDA graphs of operator applies (bdgd_set_graphs)

@@ -32,6 +32,7 @@
 #include "bdg_dev.h"
 #include "bdg_kern.cuh"
 #include "bdg_lines.h"
+#include "bdg_planes.h"
 
 static void graphs_clear(bdgd_ctx *c);
 
@@ -794,8 +795,8 @@ extern "C" int bdgd_create(bdgd_ctx **out, uint64_t dim, const uint64_t *N, cons
       cudaMemcpy(c->d_roots32[d], h32, sizeof(float2) * n, cudaMemcpyHostToDevice);
       cudaMemcpy(c->d_kx2[d], hk, sizeof(double) * n, cudaMemcpyHostToDevice);
     }
-    free(h64);
-    free(h32);
+    c->h_roots64[d] = h64;
+    c->h_roots32[d] = h32;
     free(hk);
     if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess) {
       bdgd_destroy(&c);
@@ -818,6 +819,8 @@ extern "C" void bdgd_destroy(bdgd_ctx **pc) {
     cudaFree(c->d_roots64[d]);
     cudaFree(c->d_roots32[d]);
     cudaFree(c->d_kx2[d]);
+    free(c->h_roots64[d]);
+    free(c->h_roots32[d]);
   }
   void *bufs[] = {c->ltK64, c->ltM64, c->pK64, c->pM64, c->ltK32, c->ltM32, c->pK32, c->pM32,
                   c->wf64,  c->wf32,  c->vdd,  c->ptab};
@@ -1028,15 +1031,17 @@ static int cols_ct(bdgd_ctx *c, const Prog &p, const FieldsDev &fd, typename Cx<
   return BDGD_ERR_UNSUPPORTED;
 }
 
-// FFT pass family: register line transforms (default), compile-time sized
-// shared-memory stages, or the generic runtime-sized kernels.  BDG_FFT_PATH
-// = reg | ct | generic overrides (BDG_GENERIC_FFT=1 is the same as generic).
-enum { FFT_PATH_REG = 0, FFT_PATH_CT = 1, FFT_PATH_GENERIC = 2 };
+// FFT pass family: register transforms (default; the plane passes where they
+// can run, else the line passes), compile-time sized shared-memory stages, or
+// the generic runtime-sized kernels.  BDG_FFT_PATH = reg | lines | ct | generic
+// overrides (BDG_GENERIC_FFT=1 is the same as generic).
+enum { FFT_PATH_REG = 0, FFT_PATH_CT = 1, FFT_PATH_GENERIC = 2, FFT_PATH_LINES = 3 };
 static int fft_path(const bdgd_ctx *c) {
-  if (c->force_path) return c->force_path == 2 ? FFT_PATH_CT : FFT_PATH_REG;
+  if (c->force_path) return c->force_path == 2 ? FFT_PATH_CT : c->force_path == 3 ? FFT_PATH_LINES : FFT_PATH_REG;
   if (getenv("BDG_GENERIC_FFT")) return FFT_PATH_GENERIC;
   const char *e = getenv("BDG_FFT_PATH");
   if (e) {
+    if (!strcmp(e, "lines")) return FFT_PATH_LINES;
     if (!strcmp(e, "ct")) return FFT_PATH_CT;
     if (!strcmp(e, "generic")) return FFT_PATH_GENERIC;
   }
@@ -1077,6 +1082,8 @@ static int run_program(bdgd_ctx *c, const Prog &p, const void *x, long long ldx,
   }
   // column chunking bounded by the scratch cap
   const size_t per_col = sizeof(C) * (size_t)p.J * (size_t)g.H;
+  const bool planes = !only_fwd && !only_bwd && fft_path(c) == FFT_PATH_REG &&
+                      bdgd_planes_usable(c, f32 ? BDGD_F32 : BDGD_F64);
   int chunk = ncol;
   if (per_col * (size_t)chunk > c->spec_cap) {
     chunk = (int)(c->spec_cap / per_col);
@@ -1089,7 +1096,19 @@ static int run_program(bdgd_ctx *c, const Prog &p, const void *x, long long ldx,
   if (c->spec != spec_before) c->version++;  // captured graphs hold the old scratch
   C *spec = (C *)c->spec;
   const int tx = f32 ? 16 : 8;
-  if (!only_fwd && !only_bwd && fft_path(c) == FFT_PATH_REG && bdgd_lines_usable(c, p)) {
+  if (planes) {
+    for (int c0 = 0; c0 < ncol; c0 += chunk) {
+      const int nc = (ncol - c0) < chunk ? (ncol - c0) : chunk;
+      const size_t esz = CPLX ? sizeof(C) : sizeof(T);
+      const void *xc = (const char *)x + (size_t)c0 * ldx * esz;
+      void *yc = (char *)y + (size_t)c0 * ldy * esz;
+      const int rc = f32 ? bdgd_planes_apply_f32(c, p, fd, xc, ldx, yc, ldy, spec, nc)
+                         : bdgd_planes_apply_f64(c, p, fd, xc, ldx, yc, ldy, spec, nc);
+      if (rc) return rc;
+    }
+    return BDGD_OK;
+  }
+  if (!only_fwd && !only_bwd && (fft_path(c) == FFT_PATH_REG || fft_path(c) == FFT_PATH_LINES) && bdgd_lines_usable(c, p)) {
     for (int c0 = 0; c0 < ncol; c0 += chunk) {
       const int nc = (ncol - c0) < chunk ? (ncol - c0) : chunk;
       const size_t esz = CPLX ? sizeof(C) : sizeof(T);
@@ -1336,22 +1355,30 @@ static int apply_graph(bdgd_ctx *c, int op, const Prog &p, int prec, const void 
   return BDGD_OK;
 }
 
-// Choose the FFT pass family of (op, prec) on this context by timing both
-// (each run twice, the second timed) on its first apply of >= 4 columns;
-// later applies use the faster one.  BDG_FFT_PATH / BDG_GENERIC_FFT override.
+// Choose the FFT pass family of (op, prec) on this context by timing each
+// (run twice, the second timed) on its first apply of >= 4 columns; later
+// applies use the fastest.  The register family has two forms, plane passes and
+// line passes: planes win by 1.1 to 1.7 on most grids, lines by up to 1.2 where
+// z is 256 long or one FP32 complex plane fills an SM (128^3 c64: 1077 against
+// 936 us for 8 columns), so both are timed where both can run.  BDG_FFT_PATH /
+// BDG_GENERIC_FFT override.
 static int apply_tuned(bdgd_ctx *c, int op, const Prog &p, int prec, const void *x, long long ldx, void *y,
                        long long ldy, int ncol) {
   const int pi = prec == BDGD_F32 ? 1 : 0;
   const bool env = getenv("BDG_FFT_PATH") || getenv("BDG_GENERIC_FFT");
   const bool tunable = !env && bdgd_lines_usable(c, p) && op < 16;
   if (tunable && c->tune[op][pi] == 0 && ncol >= 4 && !bdgd_capturing) {
-    float ms[2] = {0.f, 0.f};
+    // force_path: 1 plane passes, 2 shared-memory stages, 3 line passes
+    float ms[4] = {0.f, 0.f, 0.f, 0.f};
+    const bool planes = bdgd_planes_usable(c, prec);
+    const int order[3] = {2, planes ? 3 : 1, 1};  // the likely choice last: its result stays in y
     cudaEvent_t e0, e1;
     BDGD_CK(cudaEventCreate(&e0));
     BDGD_CK(cudaEventCreate(&e1));
     int rc = BDGD_OK;
-    for (int k = 0; k < 2 && !rc; ++k) {
-      c->force_path = k + 1;
+    for (int i = 0; i < (planes ? 3 : 2) && !rc; ++i) {
+      const int k = order[i];
+      c->force_path = k;
       rc = dispatch(c, p, prec, x, ldx, y, ldy, ncol, 0, 0);
       if (!rc) {
         cudaEventRecord(e0, c->stream);
@@ -1366,12 +1393,14 @@ static int apply_tuned(bdgd_ctx *c, int op, const Prog &p, int prec, const void 
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (rc) return rc;
-    c->tune[op][pi] = ms[0] <= ms[1] ? 1 : 2;
-    c->tune_ms[op][pi][0] = ms[0];
-    c->tune_ms[op][pi][1] = ms[1];
+    c->tune_lines[op][pi] = planes && ms[3] < ms[1];
+    const float reg = c->tune_lines[op][pi] ? ms[3] : ms[1];
+    c->tune[op][pi] = reg <= ms[2] ? 1 : 2;
+    c->tune_ms[op][pi][0] = reg;
+    c->tune_ms[op][pi][1] = ms[2];
     return BDGD_OK;  // y holds the result of the last run
   }
-  if (tunable && c->tune[op][pi]) c->force_path = c->tune[op][pi];
+  if (tunable && c->tune[op][pi]) c->force_path = c->tune[op][pi] == 1 && c->tune_lines[op][pi] ? 3 : c->tune[op][pi];
   const int rc = (c->graphs_on && !bdgd_capturing) ? apply_graph(c, op, p, prec, x, ldx, y, ldy, ncol)
                                                    : dispatch(c, p, prec, x, ldx, y, ldy, ncol, 0, 0);
   c->force_path = 0;

@@ -94,7 +94,7 @@ int bdgd_set_graphs(bdgd_ctx *ctx, int on);
 int bdgd_trim(bdgd_ctx *ctx);
 
 /* FFT pass family the autotuner chose for (op, prec) on this context: 0 not
- * tuned yet, 1 register-resident line transforms, 2 compile-time
+ * tuned yet, 1 register-resident transforms (planes or lines), 2 compile-time
  * shared-memory stages; ms_out (2 floats, may be NULL) receives the timed
  * milliseconds of both.  Tuning happens on the first apply of >= 4 columns
  * unless BDG_FFT_PATH or BDG_GENERIC_FFT fixes the family. */
