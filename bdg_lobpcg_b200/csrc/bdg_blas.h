@@ -3,6 +3,7 @@
 #ifndef BDG_BLAS_H
 #define BDG_BLAS_H
 
+#include <stddef.h>
 #include <stdint.h>
 
 #include "bdg/bdg_cuda.h"
@@ -29,6 +30,20 @@ int bdgd_gather_cols(bdgd_ctx *c, const double *In, int ldi, int rows, const int
                      double *Out, int ldo);
 int bdgd_scale_cols(bdgd_ctx *c, const double *In, int rows, int col0, int ncols, int cplx, const double *rowscale,
                     const double *colval, int invsqrt, int reverse, double *Out);
+/* Z (k x k upper triangular, column-major, leading dimension k) with
+ * Z^T G Z = I from the Cholesky factor of the symmetric G (leading dimension
+ * ldg; unit diagonal by scaling); *d_minpiv (device) is the smallest pivot of
+ * the scaled G, <= 0 when it is not positive definite.  Real, k at most
+ * BDGD_CHOL_MAX, else BDGD_ERR_UNSUPPORTED. */
+#define BDGD_CHOL_MAX 192
+int bdgd_chol_inverse(bdgd_ctx *c, const double *G, int k, int ldg, double *Z, double *d_minpiv);
+/* All eigenvalues (w, ascending) of the symmetric A (k x k, column-major, not
+ * changed) and unit eigenvectors Y (k x nv) of the nv largest, those of close
+ * eigenvalues not orthogonal to each other (bdg_eig.cu); *d_check the largest
+ * residual relative to ||A||.  work: bdgd_eig_work(k, nv) bytes.  3 <= k <= 192,
+ * else BDGD_ERR_UNSUPPORTED. */
+size_t bdgd_eig_work(int k, int nv);
+int bdgd_eig_top(bdgd_ctx *c, const double *A, int k, int nv, double *w, double *Y, double *work, double *d_check);
 int bdgd_hermitize(bdgd_ctx *c, double *A, int k, int cplx);
 int bdgd_clamp(bdgd_ctx *c, double *w, int n, double floor_rel);
 

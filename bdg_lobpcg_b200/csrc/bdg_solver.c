@@ -48,6 +48,11 @@
 
 #define DROP_F64 1e-13
 #define DROP_F32 1e-7
+#define EIG_PIV 1e-6 /* inverse iteration: smallest pivot of its vectors' Gram matrix */
+#define EIG_RES 1e-13 /* and their largest residual, relative to the norm */
+#define THETA_SPREAD 1e4 /* largest over m-th largest theta: above it the pencil is solved graded */
+#define PIV_F64 1e-6
+#define PIV_F32 1e-3
 #define CLAMP_A 1e-14
 /* Guard columns (nev..m-1) stay active while their backward error exceeds
  * the guard level: GUARD_LOCK while the worst backward error of the
@@ -78,12 +83,13 @@ typedef struct {
   /* small dense (FP64, device) */
   int K;         /* 3m */
   double *gout;  /* 3 Gram outputs, K x K */
-  double *Gs, *Gb, *Ga, *Z, *Ya, *Hh, *V, *C, *Cs, *T1s, *T2s, *dsc, *wG, *wA, *wH, *wtmp, *lam_d, *work, *norms;
+  double *Gs, *Gb, *Ga, *Z, *Ya, *Hh, *V, *C, *Cs, *T1s, *T2s, *dsc, *wG, *wA, *wH, *wtmp, *lam_d, *work, *norms, *piv, *eigw;
   float *C32;
   int *colmap, *actcols;
   double *defl;  /* psi0 and w = M^-1 psi0 (block precision), n_half each */
   double wpsi;   /* w^H psi0 */
   int deflate;
+  int graded;    /* the Rayleigh-Ritz steps of this loop take the eigen-decompositions */
   cublasHandle_t blas;
   cusolverDnHandle_t sol;
   void *swork;
@@ -112,7 +118,7 @@ static void ws_free(ws_t *w) {
   for (int i = 0; i < NB_COUNT; i++)
     if (w->blk[i]) dfree(w, w->blk[i]);
   void *bufs[] = {w->TR, w->gout, w->Gs, w->Gb, w->Ga, w->Z, w->Ya, w->Hh, w->V, w->C, w->Cs, w->T1s, w->T2s,
-                  w->dsc, w->wG, w->wA, w->wH, w->wtmp, w->lam_d, w->work, w->norms, w->C32, w->colmap,
+                  w->dsc, w->wG, w->wA, w->wH, w->wtmp, w->lam_d, w->work, w->norms, w->piv, w->eigw, w->C32, w->colmap,
                   w->actcols, w->defl, w->swork, w->info};
   for (size_t i = 0; i < sizeof bufs / sizeof bufs[0]; i++)
     if (bufs[i]) dfree(w, bufs[i]);
@@ -394,6 +400,11 @@ static int ws_setup(ws_t *w, bdgd_ctx *dev, uint64_t S, uint64_t m, uint64_t nev
   for (size_t i = 0; i < sizeof vec / sizeof vec[0]; i++) TRY(dmalloc(w, (void **)vec[i], (size_t)w->K * sizeof(double)));
   TRY(dmalloc(w, (void **)&w->work, 2 * 64 * (size_t)w->K * sizeof(double)));
   TRY(dmalloc(w, (void **)&w->norms, 4 * (size_t)w->K * sizeof(double)));
+  TRY(dmalloc(w, (void **)&w->piv, 4 * sizeof(double)));
+  if (!cplx) {
+    const int ke = w->K < BDGD_CHOL_MAX ? w->K : BDGD_CHOL_MAX;
+    TRY(dmalloc(w, (void **)&w->eigw, bdgd_eig_work(ke, (int)m < ke ? (int)m : ke)));
+  }
   TRY(dmalloc(w, (void **)&w->colmap, (size_t)w->K * sizeof(int)));
   TRY(dmalloc(w, (void **)&w->actcols, (size_t)w->K * sizeof(int)));
   TRY(dmalloc(w, (void **)&w->info, sizeof(int)));
@@ -482,8 +493,40 @@ static int scaled_eig(ws_t *w, bdgd_ctx *dev, const double *G, int k, int ldg, d
   return 0;
 }
 
-/* Z (k x keep) with Z^H G Z = I: SVQB coefficients. */
+/* Z (k x k) with Z^H G Z = I from the Cholesky factor of G, *ok = 0 where the
+ * eigen-decomposition has to decide instead: complex blocks, k above the
+ * kernel's size, or a pivot of the scaled G below PIV_F64 / PIV_F32.  There Z
+ * would amplify the rounding of G by 1/pivot; the eigen-decomposition keeps
+ * directions down to DROP_*, whose rounding is amplified likewise, but can
+ * drop those below.  One kernel against a chain of syevd launches: 0.02 against
+ * 1.2 ms at k = 96.  BDG_SMALL_EIG=1 takes the eigen-decomposition always. */
+static int chol_launch(ws_t *w, bdgd_ctx *dev, const double *G, int k, int ldg, double *Z, int *launched) {
+  const char *e = getenv("BDG_SMALL_EIG");
+  *launched = 0;
+  if (w->cplx || k > BDGD_CHOL_MAX || (e && e[0] == '1')) return 0;
+  DEV_TRY(bdgd_chol_inverse(dev, G, k, ldg, Z, w->piv));
+  *launched = 1;
+  return 0;
+}
+
+static int chol_good(const ws_t *w, double piv) { return piv >= (w->prec == BDGD_F32 ? PIV_F32 : PIV_F64); }
+
+static int chol_coef(ws_t *w, bdgd_ctx *dev, const double *G, int k, int ldg, double *Z, int *ok) {
+  TRY(chol_launch(w, dev, G, k, ldg, Z, ok));
+  if (*ok) {
+    double piv = 0.0;
+    TRY(host_vec(w, dev, w->piv, 1, &piv));
+    *ok = chol_good(w, piv);
+  }
+  return 0;
+}
+
+/* Z (k x keep) with Z^H G Z = I: Cholesky or SVQB coefficients. */
 static int svqb(ws_t *w, bdgd_ctx *dev, const double *G, int k, int ldg, double drop, double *Zout, int *keep) {
+  int ok = 0;
+  TRY(chol_coef(w, dev, G, k, ldg, Zout, &ok));
+  *keep = k;
+  if (ok) return 0;
   TRY(scaled_eig(w, dev, G, k, ldg, drop, keep));
   DEV_TRY(bdgd_scale_cols(dev, w->Gs, k, k - *keep, *keep, w->cplx, w->dsc, w->wG, 1, 0, Zout));
   return 0;
@@ -492,14 +535,17 @@ static int svqb(ws_t *w, bdgd_ctx *dev, const double *G, int k, int ldg, double 
 /* Y = G^+ Bm  (G: k x k Gram, Bm: k x q, both leading dim ld), into Yout (k x q, ld k). */
 static int gram_pinv_apply(ws_t *w, bdgd_ctx *dev, const double *G, int k, int ld, const double *Bm, int q,
                            double drop, double *Yout) {
-  int keep = 0;
-  TRY(scaled_eig(w, dev, G, k, ld, drop, &keep));
-  if (keep == 0 || q == 0) {
-    CUDA_TRY(cudaMemsetAsync(Yout, 0, (size_t)k * q * (w->cplx ? 2 : 1) * sizeof(double), stream_of(dev)));
-    return 0;
+  int keep = k, ok = 0;
+  TRY(chol_coef(w, dev, G, k, ld, w->Z, &ok));
+  if (!ok) {
+    TRY(scaled_eig(w, dev, G, k, ld, drop, &keep));
+    if (keep == 0 || q == 0) {
+      CUDA_TRY(cudaMemsetAsync(Yout, 0, (size_t)k * q * (w->cplx ? 2 : 1) * sizeof(double), stream_of(dev)));
+      return 0;
+    }
+    /* U = D Q_keep s^-1/2 ; Y = U U^H Bm */
+    DEV_TRY(bdgd_scale_cols(dev, w->Gs, k, k - keep, keep, w->cplx, w->dsc, w->wG, 1, 0, w->Z));
   }
-  /* U = D Q_keep s^-1/2 ; Y = U U^H Bm */
-  DEV_TRY(bdgd_scale_cols(dev, w->Gs, k, k - keep, keep, w->cplx, w->dsc, w->wG, 1, 0, w->Z));
   TRY(zgemm_small(w, 1, 0, keep, q, k, 1.0, w->Z, k, Bm, ld, 0.0, w->T1s, keep));
   TRY(zgemm_small(w, 0, 0, k, q, keep, 1.0, w->Z, k, w->T1s, keep, 0.0, Yout, k));
   return 0;
@@ -627,6 +673,33 @@ static int rr_grams(ws_t *w, bdgd_ctx *dev, int nb, void *const *Sb, void *const
   return 0;
 }
 
+/* Eigenvalues of the symmetric H (k x k) into w->wH, ascending, and the
+ * eigenvectors of the m largest into w->V (k x m), on the library's own
+ * kernels (k at most BDGD_CHOL_MAX; *launched = 0 otherwise).  Inverse iteration
+ * gives the vectors, their Cholesky factor orthonormalises those of close
+ * values: w->piv[1] is its smallest pivot and w->piv[2] the largest residual
+ * relative to ||H||, which the caller checks.  0.16 against 1.15 ms (syevd) at
+ * k = 96.  BDG_SMALL_EIG=2 leaves H to syevd. */
+static int eig_top_launch(ws_t *w, bdgd_ctx *dev, const double *H, int k, int m, int *launched) {
+  const char *e = getenv("BDG_SMALL_EIG");
+  *launched = 0;
+  if (!w->eigw || (e && e[0] == '2') || k < m) return 0;
+  const int rc = bdgd_eig_top(dev, H, k, m, w->wH, w->V, w->eigw, w->piv + 2);
+  if (rc == BDGD_ERR_UNSUPPORTED) return 0;
+  DEV_TRY(rc);
+  /* twice: the first pass leaves eps / pivot */
+  double *from = w->V, *to = w->T2s;
+  for (int pass = 0; pass < 2; pass++) {
+    TRY(zgemm_small(w, 1, 0, m, m, k, 1.0, from, k, from, k, 0.0, w->T1s, m));
+    DEV_TRY(bdgd_chol_inverse(dev, w->T1s, m, m, w->Hh, w->piv + (pass ? 3 : 1)));
+    TRY(zgemm_small(w, 0, 0, k, m, m, 1.0, from, k, w->Hh, m, 0.0, to, k));
+    from = to;
+    to = w->V;
+  }
+  *launched = 1;
+  return 0;
+}
+
 /* Rayleigh-Ritz of the pencil on the Gram outputs (k x k): on return w->C
  * holds C (k x m, leading dim k), lam[] the m Ritz values (ascending), *nsel
  * the number of positive-type values selected. */
@@ -635,8 +708,54 @@ static int rayleigh_ritz(ws_t *w, bdgd_ctx *dev, int k, int m, double drop, doub
   const size_t es = cplx ? 2 : 1;
   const double *G = w->gout, *Gain = w->gout + (size_t)K * K * es, *Guv = w->gout + 2 * (size_t)K * K * es;
   DEV_TRY(bdgd_rr_prepare(dev, G, Gain, Guv, k, K, cplx, w->Gs, w->Gb, w->Ga, w->dsc));
-  TRY(heev(w, w->Gs, k, k, w->wG));
   double h[3 * 1024];
+  int chol = 0;
+  if (!w->graded) TRY(chol_launch(w, dev, w->Ga, k, k, w->Z, &chol));
+  if (chol) {
+    /* A_s is well conditioned nearly always: with Z^T A_s Z = I the pencil is
+     * H = Z^T B_s Z alone, one eigen-decomposition in place of three.  The
+     * smallest pivot comes back with the eigenvalues. */
+    double piv = 0.0;
+    TRY(zgemm_small(w, 0, 0, k, k, k, 1.0, w->Gb, k, w->Z, k, 0.0, w->T1s, k));
+    TRY(zgemm_small(w, 1, 0, k, k, k, 1.0, w->Z, k, w->T1s, k, 0.0, w->Ya, k));
+    DEV_TRY(bdgd_hermitize(dev, w->Ya, k, cplx));
+    /* theta and the vectors of the m largest */
+    int own = 0;
+    const double *Q = w->Ya, *th = w->wH; /* vectors and their values, the largest last */
+    int nq = k;
+    TRY(eig_top_launch(w, dev, w->Ya, k, m, &own));
+    double chk[3] = {0.0, 0.0, 0.0};
+    CUDA_TRY(cudaMemcpyAsync(chk, w->piv, sizeof chk, cudaMemcpyDeviceToHost, stream_of(dev)));
+    if (own) TRY(host_vec(w, dev, w->wH, k, h));
+    if (own && !(chk[1] >= EIG_PIV && chk[2] <= EIG_RES)) own = 0; /* H is untouched */
+    if (own) {
+      Q = w->V;
+      th = w->wH + (k - m);
+      nq = m;
+    } else {
+      TRY(heev(w, w->Ya, k, k, w->wH));
+      TRY(host_vec(w, dev, w->wH, k, h));
+    }
+    piv = chk[0];
+    /* the rounding of H is relative to its largest value: with an undeflated
+     * zero mode (theta = 1/lambda large) the other values would carry it, so
+     * the graded eigen-decompositions below serve for the rest of the solve */
+    if (k >= m && h[k - 1] > THETA_SPREAD * fabs(h[k - m])) w->graded = 1;
+    if (chol_good(w, piv) && !w->graded) {
+      int npos = 0;
+      for (int i = 0; i < k; i++)
+        if (h[i] > 0) npos++;
+      const int sel = npos < m ? npos : m;
+      *nsel = sel;
+      if (sel == 0) return 0;
+      /* C = Z Q3[:, largest theta first] diag(theta^-1/2) */
+      DEV_TRY(bdgd_scale_cols(dev, Q, k, nq - sel, sel, cplx, NULL, th, 1, 1, w->T1s));
+      TRY(zgemm_small(w, 0, 0, k, sel, k, 1.0, w->Z, k, w->T1s, k, 0.0, w->C, k));
+      for (int j = 0; j < sel; j++) lam[j] = 1.0 / h[k - 1 - j];
+      return 0;
+    }
+  }
+  TRY(heev(w, w->Gs, k, k, w->wG));
   TRY(host_vec(w, dev, w->wG, k, h));
   const double smax = h[k - 1];
   int keep = 0;
@@ -933,6 +1052,7 @@ static int run_loop(ws_t *w, bdgd_ctx *dev, bdg_t *bdg, const loop_opts_t *o, do
   double back[1024], tres[1024];
   int act[1024];
   if (m > 1024) return -8;
+  w->graded = 0;
   /* AX, Rayleigh-Ritz on span X */
   cudaEventRecord(w->ev[0], st);
   TRY(deflate_block(w, dev, B(NB_X), m));
