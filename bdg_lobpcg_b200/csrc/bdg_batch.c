@@ -25,6 +25,7 @@
 #include "bdg/bdg_learn.h"
 
 void bdg_solver_release(bdg_t *bdg);
+void bdg_solver_release_memory(bdg_t *bdg);
 
 typedef struct {
   bdg_t **p;
@@ -65,7 +66,9 @@ static void *batch_worker(void *arg) {
     rc = bdg_solve(p);
     if (b->secs) b->secs[i] = wall() - t0;
     if (b->rcs) b->rcs[i] = rc;
-    bdg_release_device_memory(p);
+    /* the library handles stay until every worker has ended (see ws_free) */
+    bdg_solver_release_memory(p);
+    if (p->ctx && p->ctx->dev) bdgd_trim(p->ctx->dev);
   }
   return NULL;
 }
@@ -90,6 +93,7 @@ int bdg_solve_batch(bdg_t **problems, int n, int concurrency, int graphs, int *r
   if (started == 0) batch_worker(&b); /* no threads available: solve here */
   for (int t = 0; t < started; ++t) pthread_join(th[t], NULL);
   free(th);
+  for (int i = 0; i < n; ++i) bdg_solver_release(problems[i]);
   pthread_mutex_destroy(&b.mu);
   int bad = 0;
   for (int i = 0; i < n; ++i)

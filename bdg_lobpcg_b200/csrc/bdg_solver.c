@@ -113,7 +113,11 @@ static void dfree(ws_t *w, void *p) {
   if (p) cudaFreeAsync(p, w->st);
 }
 
-static void ws_free(ws_t *w) {
+/* Free the workspace; its library handles only with `handles`.  Destroying them
+ * synchronises the device, and the driver crashed in that call (now and then,
+ * inside cuCtxSynchronize) while other threads' solves were running, so the
+ * workers of bdg_solve_batch leave them to the thread that joins them. */
+static void ws_free(ws_t *w, int handles) {
   if (!w) return;
   for (int i = 0; i < NB_COUNT; i++)
     if (w->blk[i]) dfree(w, w->blk[i]);
@@ -122,8 +126,8 @@ static void ws_free(ws_t *w) {
                   w->actcols, w->defl, w->swork, w->info};
   for (size_t i = 0; i < sizeof bufs / sizeof bufs[0]; i++)
     if (bufs[i]) dfree(w, bufs[i]);
-  if (w->blas) cublasDestroy(w->blas);
-  if (w->sol) cusolverDnDestroy(w->sol);
+  if (handles && w->blas) cublasDestroy(w->blas);
+  if (handles && w->sol) cusolverDnDestroy(w->sol);
   for (int i = 0; i < 12; i++)
     if (w->ev[i]) cudaEventDestroy(w->ev[i]);
   for (int i = 0; i < 2; i++) {
@@ -135,7 +139,11 @@ static void ws_free(ws_t *w) {
     if (w->st) cudaStreamSynchronize(w->st);
     cudaFreeHost(w->hX0);
   }
+  cublasHandle_t blas = handles ? NULL : w->blas;
+  cusolverDnHandle_t sol = handles ? NULL : w->sol;
   memset(w, 0, sizeof *w);
+  w->blas = blas;
+  w->sol = sol;
 }
 
 /* memcpy of a large host range by several threads: one thread copies at a
@@ -235,10 +243,19 @@ static int staged_copy(ws_t *w, void *dst, const void *src, size_t bytes, int h2
   return 0;
 }
 
+/* Free the solver's device memory and keep its library handles. */
+void bdg_solver_release_memory(bdg_t *bdg) {
+  if (bdg->solver_ws) {
+    ws_free(&((ws_t *)bdg->solver_ws)[0], 0);
+    ws_free(&((ws_t *)bdg->solver_ws)[1], 0);
+  }
+  safe_free(&bdg->block);
+}
+
 void bdg_solver_release(bdg_t *bdg) {
   if (bdg->solver_ws) {
-    ws_free(&((ws_t *)bdg->solver_ws)[0]);
-    ws_free(&((ws_t *)bdg->solver_ws)[1]);
+    ws_free(&((ws_t *)bdg->solver_ws)[0], 1);
+    ws_free(&((ws_t *)bdg->solver_ws)[1], 1);
     free(bdg->solver_ws);
     bdg->solver_ws = NULL;
   }
@@ -378,7 +395,7 @@ static int ws_setup(ws_t *w, bdgd_ctx *dev, uint64_t S, uint64_t m, uint64_t nev
     w->p = 0;
     return 0;
   }
-  ws_free(w);
+  ws_free(w, 0);
   w->st = stream_of(dev);
   w->S = S;
   w->n = 2 * S;
@@ -408,9 +425,9 @@ static int ws_setup(ws_t *w, bdgd_ctx *dev, uint64_t S, uint64_t m, uint64_t nev
   TRY(dmalloc(w, (void **)&w->colmap, (size_t)w->K * sizeof(int)));
   TRY(dmalloc(w, (void **)&w->actcols, (size_t)w->K * sizeof(int)));
   TRY(dmalloc(w, (void **)&w->info, sizeof(int)));
-  BLAS_TRY(cublasCreate(&w->blas));
+  if (!w->blas) BLAS_TRY(cublasCreate(&w->blas));
   BLAS_TRY(cublasSetStream(w->blas, stream_of(dev)));
-  SOL_TRY(cusolverDnCreate(&w->sol));
+  if (!w->sol) SOL_TRY(cusolverDnCreate(&w->sol));
   SOL_TRY(cusolverDnSetStream(w->sol, stream_of(dev)));
   int lw = 0;
   if (cplx) {
