@@ -193,6 +193,7 @@ template <typename T> struct GStageV<T, true, 1> { typedef typename GStage<T, tr
 // three blocks per SM).  At 128^3, k = 192: 24.0 against 24.6 ms for V = 1;
 // four-stage rings (8 rows at four blocks per SM, 16 rows at two) measured
 // 36.4 and 25.8 ms.
+template <typename T> struct GStageV<T, false, 4> : GStageV<T, false, 1> {};
 template <typename T> struct GStageV<T, false, 3> { typedef typename GStage<T, false>::E E; static constexpr int RK = 16, LDE = 20; };
 template <int V> constexpr int gram_nstage() { return V == 3 ? 3 : 2; }
 
@@ -608,7 +609,108 @@ __device__ __forceinline__ void gram_tile_fit(const GTask &tk, int ti, int tj, l
       }
 }
 
-// gram_tile_fit for the tile's extent: 1..4 fragments a warp cover 16..64 columns
+// One tile of at most CW = 16 or 32 columns on either side (real): the four warps
+// share a stage's rows, not the tile, so each holds all FM x FN fragments that
+// the tile needs (to 8 columns, not 16) and loads FM + FN fragments for FM FN
+// products.  Their sums are added in order through shared memory at the end of
+// the segment.
+template <typename T, int CW, int FM, int FN>
+__device__ __forceinline__ void gram_tile_rows4(const GTask &tk, int ti, int tj, long long rbeg, long long rend,
+                                                double *__restrict__ out, T *buf) {
+  constexpr int RK = 1024 / CW, LDE = RK + 4, RPC = 16 / (int)sizeof(T), CPC = RK / RPC;
+  constexpr int STG = 2 * CW * LDE;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int lr = lane & 3, lc = lane >> 2;
+  const int na = min(GT, tk.ka - ti * GT), nb = min(GT, tk.kb - tj * GT);
+  const T *A = (const T *)tk.a + (long long)ti * GT * tk.lda;
+  const T *B = (const T *)tk.b + (long long)tj * GT * tk.ldb;
+  auto stage = [&](T *sm, long long r0) {
+#pragma unroll
+    for (int q0 = 0; q0 < 2 * CW * CPC; q0 += 128) {
+      const int q = q0 + threadIdx.x;
+      const bool isb = q >= CW * CPC;
+      const int qq = isb ? q - CW * CPC : q;
+      const int c = qq / CPC, r = (qq - c * CPC) * RPC;
+      const long long left = rend - (r0 + r);
+      const int nv = left >= RPC ? RPC : left > 0 ? (int)left : 0;
+      const bool ok = c < (isb ? nb : na) && nv > 0;
+      const T *base = isb ? B : A;
+      const T *src = ok ? base + (long long)c * (isb ? tk.ldb : tk.lda) + r0 + r : base;
+      cp_async16(sm + (isb ? CW * LDE : 0) + c * LDE + r, src, ok ? nv * (int)sizeof(T) : 0);
+    }
+    cp_async_commit();
+  };
+  double acc[FM][FN][2];
+#pragma unroll
+  for (int a = 0; a < FM; ++a)
+#pragma unroll
+    for (int b = 0; b < FN; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+  const int nst = rend > rbeg ? (int)((rend - rbeg + RK - 1) / RK) : 0;
+  if (nst > 0) stage(buf, rbeg);
+  for (int s = 0; s < nst; ++s) {
+    const T *cur = buf + (s & 1) * STG;
+    if (s + 1 < nst) {
+      stage(buf + ((s + 1) & 1) * STG, rbeg + (long long)(s + 1) * RK);
+      cp_async_wait<1>();
+    } else {
+      cp_async_wait<0>();
+    }
+    __syncthreads();
+    const T *sA = cur + lc * LDE + warp * (RK / 4) + lr, *sB = sA + CW * LDE;
+#pragma unroll
+    for (int kk = 0; kk < RK / 4; kk += 4) {
+      double ar[FM], br[FN];
+#pragma unroll
+      for (int mi = 0; mi < FM; ++mi) ar[mi] = (double)sA[mi * 8 * LDE + kk];
+#pragma unroll
+      for (int nj = 0; nj < FN; ++nj) br[nj] = (double)sB[nj * 8 * LDE + kk];
+#pragma unroll
+      for (int mi = 0; mi < FM; ++mi)
+#pragma unroll
+        for (int nj = 0; nj < FN; ++nj) dmma(acc[mi][nj][0], acc[mi][nj][1], ar[mi], br[nj]);
+    }
+    __syncthreads();
+  }
+  // add the warps' sums in order: each in turn on top of the ones before
+  double *red = (double *)buf;  // [FN * 8][FM * 8 + 1]; a stage of T = float holds it too
+  for (int w = 0; w < 4; ++w) {
+    if (warp == w) {
+#pragma unroll
+      for (int mi = 0; mi < FM; ++mi)
+#pragma unroll
+        for (int nj = 0; nj < FN; ++nj)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            double *p = red + (nj * 8 + 2 * lr + e) * (FM * 8 + 1) + mi * 8 + lc;
+            const double v = (w ? *p : 0.0) + acc[mi][nj][e];
+            if (w < 3) {
+              *p = v;
+            } else {
+              const int il = mi * 8 + lc, jl = nj * 8 + 2 * lr + e;
+              if (il < na && jl < nb) out[jl * GT + il] = v;
+            }
+          }
+    }
+    __syncthreads();
+  }
+}
+
+// a tile of a list whose tiles all have at most 32 columns on either side (V = 4)
+template <typename T>
+__device__ __forceinline__ void gram_tile_narrow(const GTask &tk, int ti, int tj, long long rbeg, long long rend,
+                                                 double *__restrict__ out, T *buf) {
+  const int na = min(GT, tk.ka - ti * GT), nb = min(GT, tk.kb - tj * GT);
+  switch ((na + 7) / 8 * 8 + (nb + 7) / 8) {
+#define GROW(FM, FN, CW) case FM * 8 + FN: return gram_tile_rows4<T, CW, FM, FN>(tk, ti, tj, rbeg, rend, out, buf)
+    GROW(1, 1, 16); GROW(1, 2, 16); GROW(2, 1, 16); GROW(2, 2, 16);
+    GROW(1, 3, 32); GROW(2, 3, 32); GROW(3, 1, 32); GROW(3, 2, 32); GROW(3, 3, 32);
+    GROW(1, 4, 32); GROW(2, 4, 32); GROW(3, 4, 32); GROW(4, 1, 32); GROW(4, 2, 32); GROW(4, 3, 32);
+    default: return gram_tile_rows4<T, 32, 4, 4>(tk, ti, tj, rbeg, rend, out, buf);
+#undef GROW
+  }
+}
+
+// any other tile (V = 1): 1..4 fragments a warp cover 16..64 columns
 template <typename T>
 __device__ __forceinline__ void gram_tile_real(const GTask &tk, int ti, int tj, long long rbeg, long long rend,
                                                double *__restrict__ out, T *buf) {
@@ -629,7 +731,7 @@ __device__ __forceinline__ void gram_tile_real(const GTask &tk, int ti, int tj, 
 // threads per block of a k_gram_sk variant (V = 2 splits real and imaginary
 // accumulation over twice the warps)
 template <int V> constexpr int gram_threads() { return V == 2 ? 256 : 128; }
-template <int V> constexpr int gram_min_blocks() { return V == 1 ? 4 : V == 3 ? 3 : V == 2 ? 2 : 1; }
+template <int V> constexpr int gram_min_blocks() { return V == 1 || V == 4 ? 4 : V == 3 ? 3 : V == 2 ? 2 : 1; }
 
 template <typename T, bool CPLX, int V>
 __global__ void __launch_bounds__(gram_threads<V>(), gram_min_blocks<V>()) k_gram_sk(GArgsSK g) {
@@ -658,7 +760,8 @@ __global__ void __launch_bounds__(gram_threads<V>(), gram_min_blocks<V>()) k_gra
     const long long first = (tk.wbase + (long long)lt * tk.rowsP) / g.per;
     const int slot = g.segbase[tau] + (int)((long long)blockIdx.x - first);
     double *out = g.part + (long long)slot * GT * GT * ES;
-    if constexpr (!CPLX && V == 1) gram_tile_real<T>(tk, ti, tj, r0, r1, out, buf);
+    if constexpr (!CPLX && V == 4) gram_tile_narrow<T>(tk, ti, tj, r0, r1, out, buf);
+    else if constexpr (!CPLX && V == 1) gram_tile_real<T>(tk, ti, tj, r0, r1, out, buf);
     else gram_tile_rows<T, CPLX, V>(tk, ti, tj, r0, r1, out, buf);
     pos += seglen;
   }
@@ -666,11 +769,11 @@ __global__ void __launch_bounds__(gram_threads<V>(), gram_min_blocks<V>()) k_gra
 
 // Sum the segment partials of every tile into the output block (and its
 // mirror); symmetric tasks take the lower triangle from the upper tiles.  A
-// block takes 32 elements of a task, its eight warps every eighth segment each,
-// and adds the eight sums in order: a call of one small task has as many
+// block takes 32 elements of a task, its sixteen warps every sixteenth segment each,
+// and adds the sixteen sums in order: a call of one small task has as many
 // segments as resident blocks, and one thread walking them all took 36 us.
-__global__ void __launch_bounds__(256) k_gram_sk_reduce(GArgsSK g, int cplx, int ldo, double *__restrict__ outbuf) {
-  __shared__ double red[8][32][2];
+__global__ void __launch_bounds__(512) k_gram_sk_reduce(GArgsSK g, int cplx, int ldo, double *__restrict__ outbuf) {
+  __shared__ double red[16][32][2];
   const int es = cplx ? 2 : 1;
   const GTask &tk = g.t[blockIdx.y];
   const int kk = tk.ka * tk.kb;
@@ -687,8 +790,8 @@ __global__ void __launch_bounds__(256) k_gram_sk_reduce(GArgsSK g, int cplx, int
     const int tau = tk.tile0 + lt;
     const double *pp = g.part + (long long)((sj - tj * GT) * GT + (si - ti * GT)) * es;
     const int s1 = g.segbase[tau + 1];
-#pragma unroll 4
-    for (int sg = g.segbase[tau] + w; sg < s1; sg += 8) {
+#pragma unroll 8
+    for (int sg = g.segbase[tau] + w; sg < s1; sg += 16) {
       re += pp[(long long)sg * GT * GT * es];
       if (cplx) im += pp[(long long)sg * GT * GT * es + 1];
     }
@@ -698,7 +801,7 @@ __global__ void __launch_bounds__(256) k_gram_sk_reduce(GArgsSK g, int cplx, int
   __syncthreads();
   if (w != 0 || q >= kk) return;
 #pragma unroll
-  for (int k = 1; k < 8; ++k) {
+  for (int k = 1; k < 16; ++k) {
     re += red[k][lane][0];
     im += red[k][lane][1];
   }
@@ -782,7 +885,7 @@ static int launch_gram_sk(bdgd_ctx *c, const GArgs &ga, int cplx, int ldo, doubl
   bdgd_count_launch();
   int kkmax = 0;
   for (int i = 0; i < g.nt; ++i) kkmax = g.t[i].ka * g.t[i].kb > kkmax ? g.t[i].ka * g.t[i].kb : kkmax;
-  k_gram_sk_reduce<<<dim3((kkmax + 31) / 32, g.nt), 256, 0, c->stream>>>(g, cplx, ldo, d_out);
+  k_gram_sk_reduce<<<dim3((kkmax + 31) / 32, g.nt), 512, 0, c->stream>>>(g, cplx, ldo, d_out);
   BDGD_CK(cudaGetLastError());
   return BDGD_OK;
 }
@@ -938,7 +1041,11 @@ extern "C" int bdgd_gram_tasks(bdgd_ctx *c, int prec, int cplx, int ntask, const
     const int ring = gv ? atoi(gv) : 0;  // 3: the three-stage ring (real FP64)
     // complex FP64: real and imaginary parts on separate warps (29.8 against
     // 28.9 TF/s at 128^3, k = 192; in FP32 the one-warp form is faster)
-    if (prec == BDGD_F32) rc = cplx ? launch_gram_sk<float, true, 0>(c, g, cplx, ldo, d_out)
+    bool narrow = half && !cplx && ring != 3;  // no tile above 32 columns
+    for (int i = 0; i < ntask; ++i) narrow = narrow && tasks[i].ka <= 32 && tasks[i].kb <= 32;
+    if (narrow) rc = prec == BDGD_F32 ? launch_gram_sk<float, false, 4>(c, g, cplx, ldo, d_out)
+                                      : launch_gram_sk<double, false, 4>(c, g, cplx, ldo, d_out);
+    else if (prec == BDGD_F32) rc = cplx ? launch_gram_sk<float, true, 0>(c, g, cplx, ldo, d_out)
                               : half ? launch_gram_sk<float, false, 1>(c, g, cplx, ldo, d_out)
                                      : launch_gram_sk<float, false, 0>(c, g, cplx, ldo, d_out);
     else if (cplx) rc = half ? launch_gram_sk<double, true, 2>(c, g, cplx, ldo, d_out)
@@ -1498,6 +1605,7 @@ extern "C" int bdgd_set_ritz_block(bdgd_ctx *c, double *Ga, double *Guv, int ldo
 #define UKC 16   // contraction columns per stage
 #define ULDM 68  // S stage row: 64 rows + 4 (the 16 fragment addresses of a half-warp fall in distinct banks)
 #define ULDK 20  // C stage row: UKC + 4
+#define URES_MAX (48 * 1024)  // resident coefficients: with a three-stage ring, three blocks per SM
 
 struct UTerm {
   const double *s;
@@ -1515,6 +1623,10 @@ struct UArgs {
   long long n, ld;
   int nct;
   signed char ct_out[UMAXCT], ct_col[UMAXCT];
+  // resident coefficients: offset (doubles) and row stride of each column
+  // task's matrix in shared memory; own[ct] = 0 where an earlier task's serves
+  int res_off[UMAXCT], res_ld[UMAXCT];
+  signed char own[UMAXCT];
 };
 
 __device__ __forceinline__ void cp_async8(void *smem, const void *gmem, int src_bytes) {
@@ -1522,13 +1634,13 @@ __device__ __forceinline__ void cp_async8(void *smem, const void *gmem, int src_
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gmem), "r"(src_bytes));
 }
 
-// fragments of 8 output columns per warp (two warps side by side) that cover n
-// of the 64 columns of a tile
-__device__ __forceinline__ int upd_frags(int n) { return n >= 64 ? 4 : (n + 15) / 16; }
+// fragments of 8 that cover n of the 64 output columns of a tile; above 48 all 8
+__device__ __forceinline__ int upd_frags(int n) { return n > 48 ? 8 : (n + 7) / 8; }
 
 // stage j of term tm: S columns [UKC j, UKC j + UKC) of rows [r0, r0 + 64) as
 // sA[column][row], and the matching UKC rows of C for output columns
 // [c0, c0 + 64) as sB[output column][k]; out-of-range entries are zero-filled
+template <bool RES>
 __device__ __forceinline__ void upd_stage(double *sA, double *sB, const UTerm &tm, int j, long long r0, long long n,
                                           long long ld, int c0, int ncol) {
   const int kc0 = UKC * j;
@@ -1541,8 +1653,9 @@ __device__ __forceinline__ void upd_stage(double *sA, double *sB, const UTerm &t
     const double *src = ok ? tm.s + (long long)(kc0 + col) * ld + row : tm.s;
     cp_async16(sA + col * ULDM + 2 * ch, src, ok ? (int)(nv * 8) : 0);
   }
+  if (RES) return;
   // only the output columns that the tile's fragments cover
-  const int nbc = upd_frags(ncol - c0) * 16;
+  const int nbc = upd_frags(ncol - c0) * 8;
   for (int q = threadIdx.x; q < nbc * UKC; q += 128) {
     const int oc = q / UKC, kk = q % UKC;
     const bool ok = (c0 + oc) < ncol && (kc0 + kk) < tm.k;
@@ -1566,11 +1679,15 @@ __device__ __forceinline__ int upd_nst(const UArgs &u, int ct) {
 // previous tile's last products and its stores.
 // With beta != 0 the accumulators start at (beta / alpha) Y, loaded together
 // at the start of the tile (exact for the solver's alpha = +-1, beta = 1).
-template <int USTG, int MINB>
+// RES: the small matrices stay in shared memory (loaded once by each block), so a
+// stage copies S alone: at 32 columns half of a stage's copies were 8-byte ones of
+// C, and the issue slots they took held DMMA at 54%.  Taken where the matrices
+// fit beside the ring at three blocks per SM.
+template <int USTG, int MINB, bool RES>
 __global__ void __launch_bounds__(128, MINB) k_block_update(UArgs u, long long nrt) {
   extern __shared__ __align__(16) unsigned char usm[];
   double *buf = (double *)usm;  // [USTG][A: UKC x ULDM | B: 64 x ULDK]
-  constexpr int STG = UKC * ULDM + 64 * ULDK;
+  constexpr int STG = UKC * ULDM + (RES ? 0 : 64 * ULDK);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int wi = warp & 1, wj = warp >> 1;
   const int lr = lane & 3, lc = lane >> 2;
@@ -1582,7 +1699,7 @@ __global__ void __launch_bounds__(128, MINB) k_block_update(UArgs u, long long n
     if (lrt < nrt) {
       const UOut &o = u.o[u.ct_out[lct]];
       double *dst = buf + slot * STG;
-      upd_stage(dst, dst + UKC * ULDM, o.t[lb], lj, lrt * 64, u.n, u.ld, 64 * u.ct_col[lct], o.ncol);
+      upd_stage<RES>(dst, dst + UKC * ULDM, o.t[lb], lj, lrt * 64, u.n, u.ld, 64 * u.ct_col[lct], o.ncol);
       if (++lj == (o.t[lb].k + UKC - 1) / UKC) {
         lj = 0;
         if (++lb == o.nterm) {
@@ -1595,34 +1712,58 @@ __global__ void __launch_bounds__(128, MINB) k_block_update(UArgs u, long long n
   };
 #pragma unroll
   for (int q = 0; q < USTG - 1; ++q) issue(q);
+  if constexpr (RES) {
+    // C of column task ct as [output column][k], each term padded to whole stages
+    for (int ct = 0; ct < u.nct; ++ct) {
+      if (!u.own[ct]) continue;
+      const UOut &o = u.o[u.ct_out[ct]];
+      const int c0 = 64 * u.ct_col[ct], nc = upd_frags(o.ncol - c0) * 8;
+      double *m = buf + USTG * STG + u.res_off[ct];
+      int k0 = 0;
+      for (int b = 0; b < o.nterm; ++b) {
+        const UTerm &t = o.t[b];
+        const int kp = (t.k + UKC - 1) / UKC * UKC;
+        for (int q = threadIdx.x; q < nc * kp; q += 128) {
+          const int oc = q / kp, kk = q - oc * kp;
+          m[oc * u.res_ld[ct] + k0 + kk] =
+              c0 + oc < o.ncol && kk < t.k ? __ldg(t.c + (long long)(c0 + oc) * t.ldc + kk) : 0.0;
+        }
+        k0 += kp;
+      }
+    }
+    __syncthreads();
+  }
   int slot = 0;
-  // one output tile with FN fragments of 8 columns per warp: the blocks of a
-  // solve below sizeSub 64 fill a part of the 64 columns, and multiplying the
-  // rest doubled the time at 32 (815 against 548 us for the update of a 64^3 solve)
-  auto tile = [&](auto FNC, long long rt, int ct) {
-    constexpr int FN = decltype(FNC)::value;
+  // one output tile of NF fragments of 8 columns.  64 columns: four warps of 32 x
+  // 32.  Fewer (blocks of a solve below sizeSub 64): four warps of 16 rows and all
+  // NF fragments, so no column beyond the next multiple of 8 is multiplied
+  auto tile = [&](auto NFC, long long rt, int ct) {
+    constexpr int NF = decltype(NFC)::value;
+    constexpr bool WIDE = NF == 8;
+    constexpr int FM = WIDE ? 4 : 2, FN = WIDE ? 4 : NF;
+    const int rw = WIDE ? wi * 32 : warp * 16, cw = WIDE ? wj * 32 : 0;
     const long long r0 = rt * 64;
     const UOut &o = u.o[u.ct_out[ct]];
     const int c0 = 64 * u.ct_col[ct];
     const int nst = upd_nst(u, ct);
     const double alpha = o.alpha, beta = o.beta;
     double *y = o.y;
-    double acc[4][FN][2];
+    double acc[FM][FN][2];
     if (beta != 0.0) {
       const double sc = beta / alpha;
 #pragma unroll
-      for (int mi = 0; mi < 4; ++mi)
+      for (int mi = 0; mi < FM; ++mi)
 #pragma unroll
         for (int nj = 0; nj < FN; ++nj)
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            const long long row = r0 + wi * 32 + mi * 8 + lc;
-            const int col = c0 + (wj * FN + nj) * 8 + 2 * lr + e;
+            const long long row = r0 + rw + mi * 8 + lc;
+            const int col = c0 + cw + nj * 8 + 2 * lr + e;
             acc[mi][nj][e] = (row < u.n && col < o.ncol) ? sc * __ldcs(y + (long long)col * u.ld + row) : 0.0;
           }
     } else {
 #pragma unroll
-      for (int mi = 0; mi < 4; ++mi)
+      for (int mi = 0; mi < FM; ++mi)
 #pragma unroll
         for (int nj = 0; nj < FN; ++nj) acc[mi][nj][0] = acc[mi][nj][1] = 0.0;
     }
@@ -1630,73 +1771,102 @@ __global__ void __launch_bounds__(128, MINB) k_block_update(UArgs u, long long n
       cp_async_wait<USTG - 2>();
       __syncthreads();  // stage `slot` visible to all; the slot refilled below is no longer read
       issue((slot + USTG - 1) % USTG);
-      const double *sA = buf + slot * STG, *sB = sA + UKC * ULDM;
+      const double *sA = buf + slot * STG;
+      const int ldk = RES ? u.res_ld[ct] : ULDK;
+      const double *sB = (RES ? buf + USTG * STG + u.res_off[ct] + UKC * s : sA + UKC * ULDM) + (cw + lc) * ldk + lr;
 #pragma unroll
       for (int kk = 0; kk < UKC; kk += 4) {
-        double ar[4], br[FN];
+        double ar[FM], br[FN];
 #pragma unroll
-        for (int mi = 0; mi < 4; ++mi) ar[mi] = sA[(kk + lr) * ULDM + wi * 32 + mi * 8 + lc];
+        for (int mi = 0; mi < FM; ++mi) ar[mi] = sA[(kk + lr) * ULDM + rw + mi * 8 + lc];
 #pragma unroll
-        for (int nj = 0; nj < FN; ++nj) br[nj] = sB[((wj * FN + nj) * 8 + lc) * ULDK + kk + lr];
+        for (int nj = 0; nj < FN; ++nj) br[nj] = sB[nj * 8 * ldk + kk];
 #pragma unroll
-        for (int mi = 0; mi < 4; ++mi)
+        for (int mi = 0; mi < FM; ++mi)
 #pragma unroll
           for (int nj = 0; nj < FN; ++nj) dmma(acc[mi][nj][0], acc[mi][nj][1], ar[mi], br[nj]);
       }
       slot = slot == USTG - 1 ? 0 : slot + 1;
     }
 #pragma unroll
-    for (int mi = 0; mi < 4; ++mi)
+    for (int mi = 0; mi < FM; ++mi)
 #pragma unroll
       for (int nj = 0; nj < FN; ++nj)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          const long long row = r0 + wi * 32 + mi * 8 + lc;
-          const int col = c0 + (wj * FN + nj) * 8 + 2 * lr + e;
+          const long long row = r0 + rw + mi * 8 + lc;
+          const int col = c0 + cw + nj * 8 + 2 * lr + e;
           if (row < u.n && col < o.ncol) __stcs(y + (long long)col * u.ld + row, alpha * acc[mi][nj][e]);
         }
   };
   for (long long rt = blockIdx.x; rt < nrt; rt += gridDim.x)
     for (int ct = 0; ct < u.nct; ++ct) {
       switch (upd_frags(u.o[u.ct_out[ct]].ncol - 64 * u.ct_col[ct])) {
-        case 1: tile(std::integral_constant<int, 1>{}, rt, ct); break;
-        case 2: tile(std::integral_constant<int, 2>{}, rt, ct); break;
-        case 3: tile(std::integral_constant<int, 3>{}, rt, ct); break;
-        default: tile(std::integral_constant<int, 4>{}, rt, ct); break;
+#define UTILE(NF) case NF: tile(std::integral_constant<int, NF>{}, rt, ct); break
+        UTILE(1); UTILE(2); UTILE(3); UTILE(4); UTILE(5); UTILE(6);
+        default: tile(std::integral_constant<int, 8>{}, rt, ct); break;
+#undef UTILE
       }
     }
   cp_async_wait<0>();
 }
 
 // resident blocks of a k_block_update variant on this device (queried once per device)
-template <int USTG, int MINB>
-static int upd_slots(size_t sm) {
-  static std::atomic<int> cache[64];  // written by several solver threads: idempotent, atomic
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) dev = 0;
-  if (cache[dev].load(std::memory_order_relaxed) <= 0) {
-    int nb = 0, nsm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_block_update<USTG, MINB>, 128, sm) != cudaSuccess ||
-        nb < 1)
-      nb = 1;
-    if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || nsm < 1) nsm = 148;
-    cache[dev].store(nb * nsm, std::memory_order_relaxed);
-  }
-  return cache[dev].load(std::memory_order_relaxed);
-}
-
-template <int USTG, int MINB>
-static int launch_update(bdgd_ctx *c, const UArgs &u, long long nrt) {
-  const size_t sm = sizeof(double) * USTG * (UKC * ULDM + 64 * ULDK);
+template <int USTG, int MINB, bool RES>
+static int launch_update(bdgd_ctx *c, const UArgs &u, long long nrt, size_t res_bytes) {
+  const size_t sm = sizeof(double) * USTG * (UKC * ULDM + (RES ? 0 : 64 * ULDK)) + res_bytes;
+  const size_t most = RES ? sizeof(double) * USTG * UKC * ULDM + URES_MAX : sm;
   if (!bdgd_capturing)
-    BDGD_CK(cudaFuncSetAttribute(k_block_update<USTG, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  const long long slots = upd_slots<USTG, MINB>(sm);
+    BDGD_CK(cudaFuncSetAttribute(k_block_update<USTG, MINB, RES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+  // resident blocks on this device, at the most shared memory that a launch
+  // takes (queried once; written by several solver threads: idempotent, atomic)
+  static std::atomic<int> cache[64];
+  const int dev = c->device >= 0 && c->device < 64 ? c->device : 0;
+  int slots = cache[dev].load(std::memory_order_relaxed);
+  if (slots <= 0) {
+    int nb = 0, nsm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_block_update<USTG, MINB, RES>, 128, most) != cudaSuccess || nb < 1)
+      nb = 1;
+    if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess || nsm < 1) nsm = 148;
+    cudaGetLastError();
+    slots = nb * nsm;
+    cache[dev].store(slots, std::memory_order_relaxed);
+  }
   const long long nblk = nrt < slots ? nrt : slots;
   bdgd_count_launch();
-  k_block_update<USTG, MINB><<<(unsigned)nblk, 128, sm, c->stream>>>(u, nrt);
+  k_block_update<USTG, MINB, RES><<<(unsigned)nblk, 128, sm, c->stream>>>(u, nrt);
   BDGD_CK(cudaGetLastError());
   return BDGD_OK;
+}
+
+// Place every column task's coefficients in shared memory, tasks with the same
+// matrices (X and AX, P and AP) sharing one copy; returns the bytes.
+static size_t upd_residency(UArgs &u) {
+  size_t at = 0;
+  for (int ct = 0; ct < u.nct; ++ct) {
+    const UOut &o = u.o[u.ct_out[ct]];
+    int kp = 0;
+    for (int b = 0; b < o.nterm; ++b) kp += (o.t[b].k + UKC - 1) / UKC * UKC;
+    u.own[ct] = 1;
+    u.res_ld[ct] = kp + 4;
+    for (int q = 0; q < ct && u.own[ct]; ++q) {
+      const UOut &p = u.o[u.ct_out[q]];
+      bool same = u.ct_col[q] == u.ct_col[ct] && p.ncol == o.ncol && p.nterm == o.nterm;
+      for (int b = 0; same && b < o.nterm; ++b)
+        same = p.t[b].c == o.t[b].c && p.t[b].k == o.t[b].k && p.t[b].ldc == o.t[b].ldc;
+      if (same) {
+        u.own[ct] = 0;
+        u.res_off[ct] = u.res_off[q];
+      }
+    }
+    if (u.own[ct]) {
+      const int left = o.ncol - 64 * u.ct_col[ct];
+      const int nc = left > 48 ? 64 : (left + 7) / 8 * 8;
+      u.res_off[ct] = (int)at;
+      at += (size_t)nc * u.res_ld[ct];
+    }
+  }
+  return at * sizeof(double);
 }
 
 extern "C" int bdgd_block_update_oz(bdgd_ctx *c, uint64_t n, uint64_t ld, int nout, const bdgd_update_out *outs);
@@ -1754,6 +1924,8 @@ extern "C" int bdgd_block_update(bdgd_ctx *c, int prec, int cplx, uint64_t n, ui
   // blocks per SM (BDG_UPDATE_VARIANT=2), although the latter times faster
   // alone (12.8 against 13.5 ms per update)
   const char *v = getenv("BDG_UPDATE_VARIANT");
-  if (v && v[0] == '2') return launch_update<2, 4>(c, u, nrt);
-  return launch_update<4, 3>(c, u, nrt);
+  if (v && v[0] == '2') return launch_update<2, 4, false>(c, u, nrt, 0);
+  const size_t res = upd_residency(u);
+  if (res <= URES_MAX && !(v && v[0] == '4')) return launch_update<3, 3, true>(c, u, nrt, res);
+  return launch_update<4, 3, false>(c, u, nrt, 0);
 }

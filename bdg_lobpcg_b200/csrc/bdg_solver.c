@@ -48,6 +48,7 @@
 
 #define DROP_F64 1e-13
 #define DROP_F32 1e-7
+#define PROJ_FUSED 32 /* projections of at most so many columns take the update kernel */
 #define EIG_PIV 1e-6 /* inverse iteration: smallest pivot of its vectors' Gram matrix */
 #define EIG_RES 1e-13 /* and their largest residual, relative to the norm */
 #define THETA_SPREAD 1e4 /* largest over m-th largest theta: above it the pencil is solved graded */
@@ -602,7 +603,9 @@ static int bgemm(ws_t *w, bdgd_ctx *dev, const void *X, int k, const double *Cm,
  * update kernel, which beats one cuBLAS GEMM per term when the outputs share
  * several terms (the basis update: 27 against 24 TF/s at 128^3); the
  * single-term projections stay on cuBLAS, faster there (23 against 16 TF/s
- * at k = 64 with beta = 1). */
+ * at k = 64 with beta = 1), but for at most PROJ_FUSED columns, where the
+ * kernel's coefficients stay in shared memory and one launch replaces two or
+ * three (Gram stage of a 64^3 solve, sizeSub 32: 93 -> 91 ms). */
 static int upd_term(bdgd_update_out *o, const void *S, int k, const double *Cm, int ldc) {
   if (k <= 0) return 0;
   bdgd_update_term *t = &o->term[o->nterm++];
@@ -624,6 +627,10 @@ static bdgd_update_out upd_out(void *Y, int ncol, double alpha, double beta) {
 }
 
 static int bupdate(ws_t *w, bdgd_ctx *dev, int fused, int nout, const bdgd_update_out *o) {
+  for (int i = 0; i < nout && !fused; ++i) {
+    if (o[i].ncol > PROJ_FUSED) break;
+    if (i == nout - 1) fused = 1;
+  }
   if (fused && !getenv("BDG_UPDATE_BLAS") && w->prec == BDGD_F64 && !w->cplx) {
     const int rc = bdgd_block_update(dev, w->prec, w->cplx, w->n, w->n, nout, o);
     if (rc != BDGD_ERR_UNSUPPORTED) {
