@@ -531,6 +531,74 @@ __device__ __forceinline__ void gram_tile_rows(const GTask &tk, int ti, int tj, 
       }
 }
 
+// Stage copies of one tile segment: CW columns of A and of B, RK = 1024 / CW rows a
+// stage.  A thread copies the same rows of every CS-th column, so its addresses
+// are one pointer a side, advanced by RK rows a stage, and only the last stage of a
+// segment looks at the row bound.  (Forming each address anew cost 15 instructions
+// a product and held DMMA at 55%.)  Columns past the block are zeroed once a
+// segment.
+template <typename T, int CW>
+struct GLoad {
+  static constexpr int RK = 1024 / CW, LDE = RK + 4, RPC = 16 / (int)sizeof(T), CPC = RK / RPC;
+  static constexpr int CS = 128 / CPC, NI = CW / CS, STG = 2 * CW * LDE;
+  const T *pa, *pb;
+  long long da, db, left;  // rows left in the segment, from this thread's first
+  int c0, na, nb, dst;
+
+  __device__ __forceinline__ GLoad(const GTask &tk, int ti, int tj, long long rbeg, long long rend, T *buf) {
+    const int r = (threadIdx.x % CPC) * RPC;
+    c0 = threadIdx.x / CPC;
+    na = min(GT, tk.ka - ti * GT);
+    nb = min(GT, tk.kb - tj * GT);
+    pa = (const T *)tk.a + ((long long)ti * GT + c0) * tk.lda + rbeg + r;
+    pb = (const T *)tk.b + ((long long)tj * GT + c0) * tk.ldb + rbeg + r;
+    da = CS * tk.lda;
+    db = CS * tk.ldb;
+    left = rend - rbeg - r;
+    dst = c0 * LDE + r;
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+#pragma unroll
+      for (int u = 0; u < RPC; ++u) {
+        if (c0 + i * CS >= na) buf[dst + i * CS * LDE + u] = buf[STG + dst + i * CS * LDE + u] = (T)0;
+        if (c0 + i * CS >= nb)
+          buf[CW * LDE + dst + i * CS * LDE + u] = buf[STG + CW * LDE + dst + i * CS * LDE + u] = (T)0;
+      }
+  }
+  // the next stage into sm
+  __device__ __forceinline__ void next(T *sm) {
+    T *d = sm + dst;
+    if (left >= RK) {  // every thread's chunk is whole (its offset within the stage is counted in left)
+#pragma unroll
+      for (int i = 0; i < NI; ++i)
+        if (c0 + i * CS < na) cp_async16(d + i * CS * LDE, pa + i * da, 16);
+#pragma unroll
+      for (int i = 0; i < NI; ++i)
+        if (c0 + i * CS < nb) cp_async16(d + CW * LDE + i * CS * LDE, pb + i * db, 16);
+    } else {
+      const int nv = left >= RPC ? RPC : left > 0 ? (int)left : 0;
+#pragma unroll
+      for (int i = 0; i < NI; ++i) {
+        if (c0 + i * CS < na) zcopy(d + i * CS * LDE, pa + i * da, nv);
+        if (c0 + i * CS < nb) zcopy(d + CW * LDE + i * CS * LDE, pb + i * db, nv);
+      }
+    }
+    pa += RK;
+    pb += RK;
+    left -= RK;
+    cp_async_commit();
+  }
+  // nv < RPC or more values, the rest of the 16 bytes zero; nothing is read for nv = 0
+  static __device__ __forceinline__ void zcopy(T *d, const T *src, int nv) {
+    if (nv > 0) {
+      cp_async16(d, src, nv * (int)sizeof(T));
+    } else {
+#pragma unroll
+      for (int u = 0; u < RPC; ++u) d[u] = (T)0;
+    }
+  }
+};
+
 // One tile of at most CW columns on either side (real): FM x FN fragments of 8 x 8
 // per warp, the least that cover the tile in 2 x 2 warps, and stages of
 // 1024 / CW rows, so that a stage of narrow blocks brings as many bytes as one
@@ -543,41 +611,24 @@ __device__ __forceinline__ void gram_tile_rows(const GTask &tk, int ti, int tj, 
 template <typename T, int CW, int FM, int FN>
 __device__ __forceinline__ void gram_tile_fit(const GTask &tk, int ti, int tj, long long rbeg, long long rend,
                                               double *__restrict__ out, T *buf) {
-  constexpr int RK = 1024 / CW, LDE = RK + 4, RPC = 16 / (int)sizeof(T), CPC = RK / RPC;
-  constexpr int STG = 2 * CW * LDE;
+  typedef GLoad<T, CW> LD;
+  constexpr int RK = LD::RK, LDE = LD::LDE, STG = LD::STG;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int wi = warp & 1, wj = (warp >> 1) & 1;
   const int lr = lane & 3, lc = lane >> 2;
-  const int na = min(GT, tk.ka - ti * GT), nb = min(GT, tk.kb - tj * GT);
-  const T *A = (const T *)tk.a + (long long)ti * GT * tk.lda;
-  const T *B = (const T *)tk.b + (long long)tj * GT * tk.ldb;
-  auto stage = [&](T *sm, long long r0) {
-#pragma unroll
-    for (int q0 = 0; q0 < 2 * CW * CPC; q0 += 128) {
-      const int q = q0 + threadIdx.x;
-      const bool isb = q >= CW * CPC;
-      const int qq = isb ? q - CW * CPC : q;
-      const int c = qq / CPC, r = (qq - c * CPC) * RPC;
-      const long long left = rend - (r0 + r);
-      const int nv = left >= RPC ? RPC : left > 0 ? (int)left : 0;
-      const bool ok = c < (isb ? nb : na) && nv > 0;
-      const T *base = isb ? B : A;
-      const T *src = ok ? base + (long long)c * (isb ? tk.ldb : tk.lda) + r0 + r : base;
-      cp_async16(sm + (isb ? CW * LDE : 0) + c * LDE + r, src, ok ? nv * (int)sizeof(T) : 0);
-    }
-    cp_async_commit();
-  };
+  LD ld(tk, ti, tj, rbeg, rend, buf);
+  const int na = ld.na, nb = ld.nb;
   double acc[FM][FN][2];
 #pragma unroll
   for (int a = 0; a < FM; ++a)
 #pragma unroll
     for (int b = 0; b < FN; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
   const int nst = rend > rbeg ? (int)((rend - rbeg + RK - 1) / RK) : 0;
-  if (nst > 0) stage(buf, rbeg);
+  if (nst > 0) ld.next(buf);
   for (int s = 0; s < nst; ++s) {
     const T *cur = buf + (s & 1) * STG;
     if (s + 1 < nst) {
-      stage(buf + ((s + 1) & 1) * STG, rbeg + (long long)(s + 1) * RK);
+      ld.next(buf + ((s + 1) & 1) * STG);
       cp_async_wait<1>();
     } else {
       cp_async_wait<0>();
@@ -617,40 +668,23 @@ __device__ __forceinline__ void gram_tile_fit(const GTask &tk, int ti, int tj, l
 template <typename T, int CW, int FM, int FN>
 __device__ __forceinline__ void gram_tile_rows4(const GTask &tk, int ti, int tj, long long rbeg, long long rend,
                                                 double *__restrict__ out, T *buf) {
-  constexpr int RK = 1024 / CW, LDE = RK + 4, RPC = 16 / (int)sizeof(T), CPC = RK / RPC;
-  constexpr int STG = 2 * CW * LDE;
+  typedef GLoad<T, CW> LD;
+  constexpr int RK = LD::RK, LDE = LD::LDE, STG = LD::STG;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int lr = lane & 3, lc = lane >> 2;
-  const int na = min(GT, tk.ka - ti * GT), nb = min(GT, tk.kb - tj * GT);
-  const T *A = (const T *)tk.a + (long long)ti * GT * tk.lda;
-  const T *B = (const T *)tk.b + (long long)tj * GT * tk.ldb;
-  auto stage = [&](T *sm, long long r0) {
-#pragma unroll
-    for (int q0 = 0; q0 < 2 * CW * CPC; q0 += 128) {
-      const int q = q0 + threadIdx.x;
-      const bool isb = q >= CW * CPC;
-      const int qq = isb ? q - CW * CPC : q;
-      const int c = qq / CPC, r = (qq - c * CPC) * RPC;
-      const long long left = rend - (r0 + r);
-      const int nv = left >= RPC ? RPC : left > 0 ? (int)left : 0;
-      const bool ok = c < (isb ? nb : na) && nv > 0;
-      const T *base = isb ? B : A;
-      const T *src = ok ? base + (long long)c * (isb ? tk.ldb : tk.lda) + r0 + r : base;
-      cp_async16(sm + (isb ? CW * LDE : 0) + c * LDE + r, src, ok ? nv * (int)sizeof(T) : 0);
-    }
-    cp_async_commit();
-  };
+  LD ld(tk, ti, tj, rbeg, rend, buf);
+  const int na = ld.na, nb = ld.nb;
   double acc[FM][FN][2];
 #pragma unroll
   for (int a = 0; a < FM; ++a)
 #pragma unroll
     for (int b = 0; b < FN; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
   const int nst = rend > rbeg ? (int)((rend - rbeg + RK - 1) / RK) : 0;
-  if (nst > 0) stage(buf, rbeg);
+  if (nst > 0) ld.next(buf);
   for (int s = 0; s < nst; ++s) {
     const T *cur = buf + (s & 1) * STG;
     if (s + 1 < nst) {
-      stage(buf + ((s + 1) & 1) * STG, rbeg + (long long)(s + 1) * RK);
+      ld.next(buf + ((s + 1) & 1) * STG);
       cp_async_wait<1>();
     } else {
       cp_async_wait<0>();
@@ -1643,15 +1677,17 @@ __device__ __forceinline__ int upd_frags(int n) { return n > 48 ? 8 : (n + 7) / 
 template <bool RES>
 __device__ __forceinline__ void upd_stage(double *sA, double *sB, const UTerm &tm, int j, long long r0, long long n,
                                           long long ld, int c0, int ncol) {
-  const int kc0 = UKC * j;
-  for (int q = threadIdx.x; q < UKC * 32; q += 128) {
-    const int col = q >> 5, ch = q & 31;
-    const long long row = r0 + 2 * ch;
-    long long nv = n - row;
-    nv = nv < 0 ? 0 : (nv > 2 ? 2 : nv);
-    const bool ok = (kc0 + col) < tm.k && nv > 0;
-    const double *src = ok ? tm.s + (long long)(kc0 + col) * ld + row : tm.s;
-    cp_async16(sA + col * ULDM + 2 * ch, src, ok ? (int)(nv * 8) : 0);
+  const int kc0 = UKC * j, col = threadIdx.x >> 5, ch = threadIdx.x & 31;
+  // a thread copies one pair of rows of every fourth column
+  const long long row = r0 + 2 * ch;
+  const int bytes = row + 2 <= n ? 16 : row < n ? 8 : 0;
+  const double *src = tm.s + (long long)(kc0 + col) * ld + row;
+  double *dst = sA + col * ULDM + 2 * ch;
+#pragma unroll
+  for (int i = 0; i < UKC / 4; ++i) {
+    const bool ok = kc0 + col + 4 * i < tm.k && bytes;
+    cp_async16(dst + 4 * i * ULDM, ok ? src : tm.s, ok ? bytes : 0);
+    src += 4 * ld;
   }
   if (RES) return;
   // only the output columns that the tile's fragments cover
