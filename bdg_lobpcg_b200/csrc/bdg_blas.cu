@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(128) k_gram_tasks2(GArgs g) {
 // segment it covers; a tile's partials are summed in a fixed order by the
 // reduction, so the result is deterministic.
 // ---------------------------------------------------------------------------
-#define GSK_STEP 32        // work-line granularity (multiple of every stage height)
+#define GSK_STEP 32        // work-line granularity (the last stage of a segment may be partial)
 #define GMAXTILES 1024
 
 struct GArgsSK {
@@ -531,16 +531,16 @@ __device__ __forceinline__ void gram_tile_rows(const GTask &tk, int ti, int tj, 
       }
 }
 
-// Stage copies of one tile segment: CW columns of A and of B, RK = 1024 / CW rows a
-// stage.  A thread copies the same rows of every CS-th column, so its addresses
+// Stage copies of one tile segment: CW columns of A and of B, RK rows a stage (elements
+// T: real, or complex as a pair).  A thread copies the same rows of every CS-th column, so its addresses
 // are one pointer a side, advanced by RK rows a stage, and only the last stage of a
 // segment looks at the row bound.  (Forming each address anew cost 15 instructions
 // a product and held DMMA at 55%.)  Columns past the block are zeroed once a
 // segment.
-template <typename T, int CW>
+template <typename T, int CW, int RKS = 1024 / CW, int LDS = RKS + 4, int THR = 128>
 struct GLoad {
-  static constexpr int RK = 1024 / CW, LDE = RK + 4, RPC = 16 / (int)sizeof(T), CPC = RK / RPC;
-  static constexpr int CS = 128 / CPC, NI = CW / CS, STG = 2 * CW * LDE;
+  static constexpr int RK = RKS, LDE = LDS, RPC = 16 / (int)sizeof(T), CPC = RK / RPC;
+  static constexpr int CS = THR / CPC, NI = CW / CS, STG = 2 * CW * LDE;
   const T *pa, *pb;
   long long da, db, left;  // rows left in the segment, from this thread's first
   int c0, na, nb, dst;
@@ -560,10 +560,15 @@ struct GLoad {
     for (int i = 0; i < NI; ++i)
 #pragma unroll
       for (int u = 0; u < RPC; ++u) {
-        if (c0 + i * CS >= na) buf[dst + i * CS * LDE + u] = buf[STG + dst + i * CS * LDE + u] = (T)0;
+        if (c0 + i * CS >= na) buf[dst + i * CS * LDE + u] = buf[STG + dst + i * CS * LDE + u] = zero();
         if (c0 + i * CS >= nb)
-          buf[CW * LDE + dst + i * CS * LDE + u] = buf[STG + CW * LDE + dst + i * CS * LDE + u] = (T)0;
+          buf[CW * LDE + dst + i * CS * LDE + u] = buf[STG + CW * LDE + dst + i * CS * LDE + u] = zero();
       }
+  }
+  static __device__ __forceinline__ T zero() {
+    T z;
+    memset(&z, 0, sizeof z);
+    return z;
   }
   // the next stage into sm
   __device__ __forceinline__ void next(T *sm) {
@@ -594,7 +599,7 @@ struct GLoad {
       cp_async16(d, src, nv * (int)sizeof(T));
     } else {
 #pragma unroll
-      for (int u = 0; u < RPC; ++u) d[u] = (T)0;
+      for (int u = 0; u < RPC; ++u) d[u] = zero();
     }
   }
 };
@@ -762,6 +767,117 @@ __device__ __forceinline__ void gram_tile_real(const GTask &tk, int ti, int tj, 
   }
 }
 
+// Complex tile: FM x FN fragments of 8 x 8 per warp in 2 x 2 warps.  SPLIT (256
+// threads): warps 0-3 sum the real parts and warps 4-7 the imaginary parts.
+template <typename T, bool SPLIT, int FM, int FN>
+__device__ __forceinline__ void gram_tile_cplx(const GTask &tk, int ti, int tj, long long rbeg, long long rend,
+                                               double *__restrict__ out, typename GStage<T, true>::E *buf) {
+  typedef typename GStage<T, true>::E E;
+  typedef GLoad<E, GT, GStage<T, true>::RK, GStage<T, true>::LDE, SPLIT ? 256 : 128> LD;
+  constexpr int RK = LD::RK, LDE = LD::LDE, STG = LD::STG;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int part = SPLIT ? warp >> 2 : 0;
+  const int wi = warp & 1, wj = (warp >> 1) & 1;
+  const int lr = lane & 3, lc = lane >> 2;
+  LD ld(tk, ti, tj, rbeg, rend, buf);
+  double acc[FM][FN][2], aci[FM][FN][2];
+#pragma unroll
+  for (int a = 0; a < FM; ++a)
+#pragma unroll
+    for (int b = 0; b < FN; ++b) acc[a][b][0] = acc[a][b][1] = aci[a][b][0] = aci[a][b][1] = 0.0;
+  const int nst = rend > rbeg ? (int)((rend - rbeg + RK - 1) / RK) : 0;
+  if (nst > 0) ld.next(buf);
+  for (int s = 0; s < nst; ++s) {
+    const E *cur = buf + (s & 1) * STG;
+    if (s + 1 < nst) {
+      ld.next(buf + ((s + 1) & 1) * STG);
+      cp_async_wait<1>();
+    } else {
+      cp_async_wait<0>();
+    }
+    __syncthreads();
+    const E *sA = cur + (wi * 8 * FM + lc) * LDE + lr, *sB = cur + (GT + wj * 8 * FN + lc) * LDE + lr;
+#pragma unroll
+    for (int kk = 0; kk < RK; kk += 4) {
+      double ar[FM], br[FN], ai[FM], bi[FN];
+#pragma unroll
+      for (int mi = 0; mi < FM; ++mi) {
+        const E v = sA[mi * 8 * LDE + kk];
+        ar[mi] = re_of<E>(v);
+        ai[mi] = im_of<E>(v);
+      }
+#pragma unroll
+      for (int nj = 0; nj < FN; ++nj) {
+        const E v = sB[nj * 8 * LDE + kk];
+        br[nj] = re_of<E>(v);
+        bi[nj] = im_of<E>(v);
+      }
+      // conj(A)^T B: re += Ar Br + Ai Bi ; im += Ar Bi - Ai Br
+      if (!SPLIT || part == 0) {
+#pragma unroll
+        for (int mi = 0; mi < FM; ++mi)
+#pragma unroll
+          for (int nj = 0; nj < FN; ++nj) {
+            dmma(acc[mi][nj][0], acc[mi][nj][1], ar[mi], br[nj]);
+            dmma(acc[mi][nj][0], acc[mi][nj][1], ai[mi], bi[nj]);
+          }
+      }
+      if constexpr (SPLIT) {
+        if (part == 1) {
+#pragma unroll
+          for (int mi = 0; mi < FM; ++mi)
+#pragma unroll
+            for (int nj = 0; nj < FN; ++nj) {
+              dmma(acc[mi][nj][0], acc[mi][nj][1], ar[mi], bi[nj]);
+              dmma(acc[mi][nj][0], acc[mi][nj][1], -ai[mi], br[nj]);
+            }
+        }
+      } else {
+#pragma unroll
+        for (int mi = 0; mi < FM; ++mi)
+#pragma unroll
+          for (int nj = 0; nj < FN; ++nj) {
+            dmma(aci[mi][nj][0], aci[mi][nj][1], ar[mi], bi[nj]);
+            dmma(aci[mi][nj][0], aci[mi][nj][1], -ai[mi], br[nj]);
+          }
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int mi = 0; mi < FM; ++mi)
+#pragma unroll
+    for (int nj = 0; nj < FN; ++nj)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int il = wi * 8 * FM + mi * 8 + lc, jl = wj * 8 * FN + nj * 8 + 2 * lr + e;
+        if (il < ld.na && jl < ld.nb) {
+          double *o = out + (jl * GT + il) * 2;
+          if constexpr (SPLIT) {
+            o[part] = acc[mi][nj][e];
+          } else {
+            o[0] = acc[mi][nj][e];
+            o[1] = aci[mi][nj][e];
+          }
+        }
+      }
+}
+
+template <typename T, bool SPLIT>
+__device__ __forceinline__ void gram_tile_cfit(const GTask &tk, int ti, int tj, long long rbeg, long long rend,
+                                               double *__restrict__ out, typename GStage<T, true>::E *buf) {
+  const int fm = (min(GT, tk.ka - ti * GT) + 15) / 16, fn = (min(GT, tk.kb - tj * GT) + 15) / 16;
+  switch (fm * 4 + fn) {
+#define GCPLX(FM, FN) case FM * 4 + FN: return gram_tile_cplx<T, SPLIT, FM, FN>(tk, ti, tj, rbeg, rend, out, buf)
+    GCPLX(1, 1); GCPLX(1, 2); GCPLX(1, 3); GCPLX(1, 4);
+    GCPLX(2, 1); GCPLX(2, 2); GCPLX(2, 3); GCPLX(2, 4);
+    GCPLX(3, 1); GCPLX(3, 2); GCPLX(3, 3); GCPLX(3, 4);
+    GCPLX(4, 1); GCPLX(4, 2); GCPLX(4, 3);
+    default: return gram_tile_cplx<T, SPLIT, 4, 4>(tk, ti, tj, rbeg, rend, out, buf);
+#undef GCPLX
+  }
+}
+
 // threads per block of a k_gram_sk variant (V = 2 splits real and imaginary
 // accumulation over twice the warps)
 template <int V> constexpr int gram_threads() { return V == 2 ? 256 : 128; }
@@ -796,6 +912,8 @@ __global__ void __launch_bounds__(gram_threads<V>(), gram_min_blocks<V>()) k_gra
     double *out = g.part + (long long)slot * GT * GT * ES;
     if constexpr (!CPLX && V == 4) gram_tile_narrow<T>(tk, ti, tj, r0, r1, out, buf);
     else if constexpr (!CPLX && V == 1) gram_tile_real<T>(tk, ti, tj, r0, r1, out, buf);
+    else if constexpr (CPLX && V == 2) gram_tile_cfit<T, true>(tk, ti, tj, r0, r1, out, buf);
+    else if constexpr (CPLX && sizeof(T) == 4) gram_tile_cfit<T, false>(tk, ti, tj, r0, r1, out, buf);
     else gram_tile_rows<T, CPLX, V>(tk, ti, tj, r0, r1, out, buf);
     pos += seglen;
   }

@@ -46,6 +46,28 @@ def test_gram_narrow_blocks(k, prec, bdg):
     dc.close()
 
 
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("k", [1, 8, 16, 17, 31, 33, 48, 64, 80])
+def test_gram_narrow_complex_blocks(k, prec, bdg):
+    torch = _torch()
+    g = torch.Generator(device="cuda").manual_seed(200 + k)
+    dt = torch.float32 if prec else torch.float64
+    dc = bdg.DeviceContext(1, [16], [1.0], True)
+    for half in (20, 1000, 4098):
+        ld = 2 * half + 4
+        S, AS = (torch.view_as_complex(torch.randn((k, ld, 2), generator=g, device="cuda", dtype=dt)) for _ in range(2))
+        out = torch.full((4, k, k), 9.0, dtype=torch.complex128, device="cuda")
+        torch.cuda.synchronize()
+        dc.gram_ptr(prec, True, half, k, S.data_ptr(), ld, AS.data_ptr(), ld, out.data_ptr())
+        dc.synchronize()
+        wide = torch.complex128
+        u, v = S[:, :half].to(wide), S[:, half:2 * half].to(wide)
+        ref = torch.stack([u @ u.conj().T, v @ v.conj().T, v @ u.conj().T,
+                           AS[:, :2 * half].to(wide) @ S[:, :2 * half].to(wide).conj().T])
+        assert float((out - ref).norm() / ref.norm()) < 1e-13, half
+    dc.close()
+
+
 @pytest.mark.parametrize("m,act", [(1, 1), (8, 7), (15, 16), (17, 16), (32, 24), (33, 31), (48, 49), (64, 63), (65, 20), (80, 66)])
 def test_update_narrow_outputs(m, act, bdg):
     torch = _torch()
