@@ -21,6 +21,8 @@ int bdgd_residual(bdgd_ctx *c, int prec, int cplx, uint64_t half, uint64_t ncol,
 int bdgd_true_residual(bdgd_ctx *c, int prec, int cplx, uint64_t half, uint64_t ncol, const void *d_KMv,
                        uint64_t ldk, const void *d_X, uint64_t ld, const double *d_lam, double *d_work,
                        double *d_tt, double *d_vv);
+/* While on, the field setters of this context do not wait for their copies. */
+void bdgd_host_apply(bdgd_ctx *c, int on);
 int bdgd_convert(bdgd_ctx *c, int to_f32, const void *src, void *dst, uint64_t n_scalars);
 int bdgd_rr_prepare(bdgd_ctx *c, const double *G, const double *Ga_in, const double *Guv, int k, int ldo, int cplx,
                     double *Gs, double *Gb, double *Ga, double *d);

@@ -18,6 +18,7 @@
 
 #include "bdg/bdg_cuda.h"
 #include "bdg/bdg_internal.h"
+#include "bdg_blas.h"
 
 #ifndef M_PI
 #define M_PI 3.14159265358979323846
@@ -186,8 +187,14 @@ int bdg_ctx_sync_device(matmul_ctx_t *ctx, int op) {
 }
 
 void bdg_ctx_apply_host(matmul_ctx_t *ctx, int op, const void *x, void *y, uint64_t ncol, const char *caller) {
+  /* the field uploads and the apply in one go: bdgd_apply_host waits for all
+   * (on an error the uploads are waited for below, before the caller's arrays
+   * are its own again) */
+  if (ctx->dev) bdgd_host_apply(ctx->dev, 1);
   int rc = bdg_ctx_sync_device(ctx, op);
   if (rc == 0) rc = bdgd_apply_host(ctx->dev, op, x, y, ncol);
+  if (ctx->dev) bdgd_host_apply(ctx->dev, 0);
+  if (rc && ctx->dev) bdgd_synchronize(ctx->dev);
   if (rc) BDG_ERROR("%s: GPU apply failed (%d): %s", caller, rc, bdgd_last_error());
 }
 

@@ -69,6 +69,8 @@ struct bdgd_ctx {
   size_t spec_bytes;
   void *io;   // staging for host applies
   size_t io_bytes;
+  void *pin;  // pinned host buffer of small host applies
+  size_t pin_bytes;
   double *gram_part;
   size_t gram_part_bytes;
   void *oz_buf;        // tensor-core Gram: column maxima of its operands + error flag (stream-ordered)
@@ -81,6 +83,7 @@ struct bdgd_ctx {
   signed char tune[16][2];
   signed char tune_lines[16][2];  // the register family runs as line passes
   float tune_ms[16][2][2];
+  int host_apply;   // inside a host apply: the setters leave the wait to its end
   int force_path;   // set while the autotuner times one family
   // CUDA graphs of operator applies (bdgd_set_graphs)
   int graphs_on;

@@ -31,6 +31,7 @@
 
 #include "bdg_dev.h"
 #include "bdg_kern.cuh"
+#include "bdg_blas.h"
 #include "bdg_lines.h"
 #include "bdg_planes.h"
 
@@ -831,6 +832,7 @@ extern "C" void bdgd_destroy(bdgd_ctx **pc) {
     if (b) cudaFreeAsync(b, c->stream);
   if (c->stream) cudaStreamSynchronize(c->stream);
   if (c->stream) cudaStreamDestroy(c->stream);
+  if (c->pin) cudaFreeHost(c->pin);
   free(c);
   *pc = nullptr;
 }
@@ -857,6 +859,13 @@ __global__ void k_ptab(GeoDev g, FieldsDev f, double *__restrict__ out) {
   }
 }
 
+// End of a setter: the caller may change its arrays.  A host apply waits once, at
+// its end, for the uploads before it too.
+static int upload_done(bdgd_ctx *c) {
+  if (!c->host_apply) BDGD_CK(cudaStreamSynchronize(c->stream));
+  return BDGD_OK;
+}
+
 static int build_ptab(bdgd_ctx *c) {
   if (!c->ptab) BDGD_CK(cudaMalloc((void **)&c->ptab, sizeof(double) * c->H));
   FieldsDev f;
@@ -869,31 +878,27 @@ static int build_ptab(bdgd_ctx *c) {
   bdgd_count_launch();
   k_ptab<<<(unsigned)blocks, 256, 0, c->stream>>>(c->geo, f, c->ptab);
   BDGD_CK(cudaGetLastError());
-  BDGD_CK(cudaStreamSynchronize(c->stream));
-  return BDGD_OK;
+  return upload_done(c);
 }
 
 // upload a host double array and its float copy
+// FP64 array and its FP32 copy, which the device rounds itself: rounding on the
+// host and a second copy took longer than the first.  No wait: upload_done().
 static int upload_pair(bdgd_ctx *c, double **d64, float **d32, const double *h, long long n) {
   if (!*d64) BDGD_CK(cudaMalloc((void **)d64, sizeof(double) * n));
   if (!*d32) BDGD_CK(cudaMalloc((void **)d32, sizeof(float) * n));
   BDGD_CK(cudaMemcpyAsync(*d64, h, sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
-  float *tmp = (float *)malloc(sizeof(float) * n);
-  for (long long i = 0; i < n; ++i) tmp[i] = (float)h[i];
-  cudaError_t e = cudaMemcpyAsync(*d32, tmp, sizeof(float) * n, cudaMemcpyHostToDevice, c->stream);
-  cudaError_t e2 = cudaStreamSynchronize(c->stream);
-  free(tmp);
-  if (e != cudaSuccess) return bdgd_check(e, "upload");
-  if (e2 != cudaSuccess) return bdgd_check(e2, "upload sync");
-  return BDGD_OK;
+  return bdgd_convert(c, 1, *d64, *d32, (uint64_t)n);
 }
+
+extern "C" void bdgd_host_apply(bdgd_ctx *c, int on) { c->host_apply = on; }
 
 extern "C" int bdgd_set_local_terms(bdgd_ctx *c, const double *ltK, const double *ltM) {
   c->version++;
   int rc;
   if (ltK && (rc = upload_pair(c, &c->ltK64, &c->ltK32, ltK, c->S))) return rc;
   if (ltM && (rc = upload_pair(c, &c->ltM64, &c->ltM32, ltM, c->S))) return rc;
-  return BDGD_OK;
+  return upload_done(c);
 }
 
 extern "C" int bdgd_set_precond(bdgd_ctx *c, const double *sK, const double *sM, double mu) {
@@ -917,7 +922,7 @@ extern "C" int bdgd_set_wavefunction(bdgd_ctx *c, const void *wf) {
   c->wf32 = d32;
   if (rc) return rc;
   c->has_wf = 1;
-  return BDGD_OK;
+  return upload_done(c);
 }
 
 extern "C" int bdgd_set_dipolar(bdgd_ctx *c, const double *vdd, double g_ddi, int enabled) {
@@ -927,7 +932,7 @@ extern "C" int bdgd_set_dipolar(bdgd_ctx *c, const double *vdd, double g_ddi, in
   if (vdd) {
     if (!c->vdd) BDGD_CK(cudaMalloc((void **)&c->vdd, sizeof(double) * c->H));
     BDGD_CK(cudaMemcpyAsync(c->vdd, vdd, sizeof(double) * c->H, cudaMemcpyHostToDevice, c->stream));
-    BDGD_CK(cudaStreamSynchronize(c->stream));
+    return upload_done(c);
   }
   return BDGD_OK;
 }
@@ -1264,6 +1269,9 @@ extern "C" int bdgd_trim(bdgd_ctx *c) {
     *bufs[i] = nullptr;
     *sizes[i] = 0;
   }
+  if (c->pin) cudaFreeHost(c->pin);
+  c->pin = nullptr;
+  c->pin_bytes = 0;
   c->version++;
   return BDGD_OK;
 }
@@ -1446,6 +1454,8 @@ extern "C" int bdgd_apply(bdgd_ctx *c, int op, int prec, const void *d_x, uint64
   return apply_tuned(c, op, p, prec, d_x, (long long)ldx, d_y, (long long)ldy, (int)ncol);
 }
 
+static const size_t kPinMax = (size_t)8 << 20;
+
 extern "C" int bdgd_apply_host(bdgd_ctx *c, int op, const void *x, void *y, uint64_t ncol) {
   const int two = (op == BDGD_OP_LREP || op == BDGD_OP_TLREP || op == BDGD_OP_SWAP) ? 2 : 1;
   const size_t esz = c->cplx ? 16 : 8;
@@ -1454,11 +1464,25 @@ extern "C" int bdgd_apply_host(bdgd_ctx *c, int op, const void *x, void *y, uint
   if (rc) return rc;
   char *dx = (char *)c->io;
   char *dy = dx + colb * ncol;
-  BDGD_CK(cudaMemcpyAsync(dx, x, colb * ncol, cudaMemcpyHostToDevice, c->stream));
+  // Small columns go through a pinned buffer of the context: the driver's own
+  // staging of pageable copies is slower, above all into pages that the caller has
+  // not touched yet (Lrep of one 32^3 column: 267 -> 225 us a call).
+  const size_t nb = colb * ncol;
+  if (nb <= kPinMax && c->pin_bytes < nb) {
+    if (c->pin) cudaFreeHost(c->pin);
+    c->pin = nullptr;
+    c->pin_bytes = 0;
+    if (cudaMallocHost(&c->pin, nb) == cudaSuccess) c->pin_bytes = nb;
+    else cudaGetLastError();
+  }
+  const bool pinned = nb <= kPinMax && c->pin_bytes >= nb;
+  if (pinned) memcpy(c->pin, x, nb);
+  BDGD_CK(cudaMemcpyAsync(dx, pinned ? c->pin : x, nb, cudaMemcpyHostToDevice, c->stream));
   rc = bdgd_apply(c, op, BDGD_F64, dx, (uint64_t)c->S * two, dy, (uint64_t)c->S * two, ncol);
   if (rc) return rc;
-  BDGD_CK(cudaMemcpyAsync(y, dy, colb * ncol, cudaMemcpyDeviceToHost, c->stream));
+  BDGD_CK(cudaMemcpyAsync(pinned ? c->pin : y, dy, nb, cudaMemcpyDeviceToHost, c->stream));
   BDGD_CK(cudaStreamSynchronize(c->stream));
+  if (pinned) memcpy(y, c->pin, nb);
   return BDGD_OK;
 }
 
