@@ -611,8 +611,7 @@ struct GLoad {
 // columns (16 times on 16) that a fitted one does.  Bound by DMMA from 48 columns
 // on, by the loads below.  With the parallel reduction: bdgd_gram at k = 48, 65536
 // rows 78 -> 45 us; the Gram stage of a 64^3 solve (32 columns) 239 -> 100 ms, of a
-// 32^3 solve (16 columns) 52 -> 23 ms; nothing changes at 64 columns (25.2 ms at
-// k = 192, 4.2 M rows).
+// 32^3 solve (16 columns) 52 -> 23 ms; nothing changed at 64 columns.
 template <typename T, int CW, int FM, int FN>
 __device__ __forceinline__ void gram_tile_fit(const GTask &tk, int ti, int tj, long long rbeg, long long rend,
                                               double *__restrict__ out, T *buf) {

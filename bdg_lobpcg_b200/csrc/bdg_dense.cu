@@ -27,9 +27,9 @@
 // with a_ij = e(i, j) and p = e(j, j) before the step.  Thread (ty, tx) of 16 x 32
 // holds the elements i = ty (mod 16), c = tx (mod 32) in registers; a step
 // exchanges one column and one row through shared memory (two buffers, so one
-// barrier a step).  Bound by the latency of the k steps: 0.3 us each at k = 96,
-// 1/p and the barrier; the 32 NB (NB + 1) / 2 multiply-adds of a thread matter
-// from k = 128 on.
+// barrier a step).  Bound by the latency of the k steps, 1/p and the barrier: 27,
+// 65 and 223 us at k = 48, 96 and 192 (0.56, 0.68 and 1.16 us a step), the
+// multiply-adds of a thread adding to it at 192.
 template <int NB>
 __global__ void __launch_bounds__(CHOL_THREADS) k_chol_inverse(const double *__restrict__ G, int k, int ldg,
                                                                double *__restrict__ Z, double *__restrict__ minpiv) {

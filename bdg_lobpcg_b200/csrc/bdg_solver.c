@@ -25,8 +25,11 @@
  *
  * Every block lives in HBM for the whole solve; per iteration the host
  * reads the Ritz values, a few small eigenvalue spectra (for the drop
- * decisions) and the residual norms.  Block updates are plain GEMMs
- * (cuBLAS); the small Hermitian eigenproblems use cuSOLVER.
+ * decisions) and the residual norms.  Real FP64 basis updates, and projections
+ * of at most PROJ_FUSED columns, run in the fused update kernel; the other block
+ * products are cuBLAS GEMMs.  The small dense work of real blocks runs on the
+ * kernels of bdg_dense.cu and bdg_eig.cu; cuSOLVER takes complex blocks, sizes
+ * above BDGD_CHOL_MAX, and the matrices that those kernels report as unfit.
  *
  * BDG_PREC_MIXED runs the same iteration with FP32 blocks and FP32 operator
  * applies (Gram accumulation and all small dense work stay FP64) until the
@@ -516,7 +519,7 @@ static int scaled_eig(ws_t *w, bdgd_ctx *dev, const double *G, int k, int ldg, d
  * kernel's size, or a pivot of the scaled G below PIV_F64 / PIV_F32.  There Z
  * would amplify the rounding of G by 1/pivot; the eigen-decomposition keeps
  * directions down to DROP_*, whose rounding is amplified likewise, but can
- * drop those below.  One kernel against a chain of syevd launches: 0.02 against
+ * drop those below.  One kernel against a chain of syevd launches: 0.065 against
  * 1.2 ms at k = 96.  BDG_SMALL_EIG=1 takes the eigen-decomposition always. */
 static int chol_launch(ws_t *w, bdgd_ctx *dev, const double *G, int k, int ldg, double *Z, int *launched) {
   const char *e = getenv("BDG_SMALL_EIG");
@@ -702,8 +705,8 @@ static int rr_grams(ws_t *w, bdgd_ctx *dev, int nb, void *const *Sb, void *const
  * kernels (k at most BDGD_CHOL_MAX; *launched = 0 otherwise).  Inverse iteration
  * gives the vectors, their Cholesky factor orthonormalises those of close
  * values: w->piv[1] is its smallest pivot and w->piv[2] the largest residual
- * relative to ||H||, which the caller checks.  0.16 against 1.15 ms (syevd) at
- * k = 96.  BDG_SMALL_EIG=2 leaves H to syevd. */
+ * relative to ||H||, which the caller checks.  bdgd_eig_top 0.26 against 1.15
+ * ms (syevd) at k = 96, m = 32.  BDG_SMALL_EIG=2 leaves H to syevd. */
 static int eig_top_launch(ws_t *w, bdgd_ctx *dev, const double *H, int k, int m, int *launched) {
   const char *e = getenv("BDG_SMALL_EIG");
   *launched = 0;
