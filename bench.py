@@ -241,6 +241,11 @@ def run_reference(args, cfg):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
         return 0
+    from oracle import ref as oracle_ref
+
+    if not os.path.exists(oracle_ref.LIB_PATH):
+        print(json.dumps({"impl": "reference", "unavailable": "oracle build missing (make -C oracle)"}))
+        return 0
     inp = reference_inputs(args, cfg)
     N = cfg["N"]
     if inp is None:
