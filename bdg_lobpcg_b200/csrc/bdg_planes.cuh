@@ -217,16 +217,22 @@ __device__ __forceinline__ void step_sync(int &tid) {
   asm volatile("" : "+r"(tid));
 }
 
+// the block's threads ask L2 for the `bytes` from p on
+template <int THR> __device__ __forceinline__ void prefetch_l2(const void *p, int bytes) {
+  for (int i = threadIdx.x * 128; i < bytes; i += THR * 128)
+    asm volatile("prefetch.global.L2 [%0];" ::"l"((const char *)p + i));
+}
+
 // ---------------------------------------------------------------------------
 // prologue, x and y forward of one plane.  grid.x: spectra (column * J +
 // job), grid.y: planes, so that blocks of all columns read a plane of the
 // coefficients together.
 // ---------------------------------------------------------------------------
-template <typename T, int MODE, typename Q>
+template <typename T, int MODE, typename Q, bool PF>
 __global__ void __launch_bounds__((plane_threads<T, Q>()), (plane_blocks<T, Q>()))
     k_plane_fwd(GeoDev g, Prog p, FieldsDev f, Q q, const __grid_constant__ TwTab<typename Cx<T>::t, Q> tw,
                 const void *__restrict__ xin, long long ldx, typename Cx<T>::t *__restrict__ spec,
-                void *__restrict__ yout, long long ldy) {
+                void *__restrict__ yout, long long ldy, int ahead) {
   typedef typename Cx<T>::t C;
   extern __shared__ __align__(16) unsigned char smraw[];
   constexpr int THR = plane_threads<T, Q>();
@@ -334,6 +340,14 @@ __global__ void __launch_bounds__((plane_threads<T, Q>()), (plane_blocks<T, Q>()
       for (int k = 0; k < R; ++k) d[k * q.x2p] = v[k];
     }
   });
+  if (PF && ahead > 0) {
+    const unsigned b = blockIdx.y * gridDim.x + blockIdx.x + ahead, zn = b / gridDim.x;
+    if (zn < gridDim.y) {
+      constexpr int es = MODE == PL_CPLX ? (int)sizeof(C) : (int)sizeof(T);
+      const int jn = b - zn * gridDim.x, cn = jn / p.J, hn = p.jh[jn - cn * p.J];
+      prefetch_l2<THR>((const char *)xin + (cn * ldx + hn * g.S + (long long)zn * q.nx * q.ny) * es, es * q.nx * q.ny);
+    }
+  }
   step_sync(tid);
   // x, second step
   step_x2(q, [&](auto RC) {
@@ -542,10 +556,10 @@ __global__ void __launch_bounds__(kZThreads, (z_blocks<T, Q>()))
 // dipolar exchange) takes two launches, the second field's first: y <- ltM x +
 // 2 g w o1, then + o0.
 // ---------------------------------------------------------------------------
-template <typename T, int MODE, typename Q>
+template <typename T, int MODE, typename Q, bool PF>
 __global__ void __launch_bounds__((plane_threads<T, Q>()), (plane_blocks<T, Q>()))
     k_plane_inv(GeoDev g, Prog p, FieldsDev f, Q q, const __grid_constant__ TwTab<typename Cx<T>::t, Q> tw,
-                const typename Cx<T>::t *__restrict__ spec, void *yout, long long ldy, int h0, int nhs, int fi) {
+                const typename Cx<T>::t *__restrict__ spec, void *yout, long long ldy, int h0, int nhs, int fi, int ahead) {
   typedef typename Cx<T>::t C;
   extern __shared__ __align__(16) unsigned char smraw[];
   constexpr int THR = plane_threads<T, Q>();
@@ -579,6 +593,18 @@ __global__ void __launch_bounds__((plane_threads<T, Q>()), (plane_blocks<T, Q>()
       for (int r = 0; r < R; ++r) d[r * rs] = v[r];
     }
   });
+  if (PF && ahead > 0) {
+    const unsigned nx = blockIdx.y * gridDim.x + blockIdx.x + ahead, zn = nx / gridDim.x;
+    if (zn < gridDim.y) {
+      const int bx = nx - zn * gridDim.x, cn = bx / nhs, hn = h0 + (bx - cn * nhs);
+      prefetch_l2<THR>(spec + ((long long)cn * p.J + p.j0[hn] + fi) * g.H + (long long)zn * q.ny * q.nxk,
+                       (int)sizeof(C) * q.ny * q.nxk);
+    }
+  }
+  if (PF && (post == POST_K || post == POST_M)) {
+    constexpr int es = MODE == PL_CPLX ? (int)sizeof(C) : (int)sizeof(T);
+    prefetch_l2<THR>((const char *)yout + (col * ldy + hf * g.S + plane) * es, es * q.nx * q.ny);
+  }
   step_sync(tid);
   // y, second step: output r of item k1 is y = k1 + yo*r
   step_ye(q, [&](auto RC) {
@@ -790,16 +816,31 @@ static int launch_after(bdgd_ctx *c, K kern, dim3 grid, int threads, size_t sm, 
   return BDGD_OK;
 }
 
-template <typename T, int MODE, typename Q, typename Qz>
-static int planes_launch(bdgd_ctx *c, const Prog &p, const FieldsDev &fd, const Q &q, const Qz &qz, const void *x,
+// Applies whose blocks and spectra together exceed kL2Bytes (what the 126 MB L2
+// keeps of data read and written once) prefetch into L2.  The inverse asks for
+// the local term in y, its epilogue's operand, before its second step; where
+// one plane fills an SM (128^3 FP64: 139 KB) nothing else hides the loads, so
+// both plane kernels also ask for the plane of the block kAhead = 148 SMs
+// later.  Without -> with: Lrep 48x64x96
+// complex 667 -> 640 us; T 128^3 FP64, 64 columns 3666 -> 3549 (the inverse's
+// lookahead alone 3560); Lrep 64^3 FP64, 32 columns 337.4 -> 335.3; Lrep 128^3
+// FP32 unchanged.  Elsewhere they cost: y below kL2Bytes 106.6 -> 107.4
+// (50x45x36, 16 columns), lookahead of both with two or more blocks an SM
+// 106.6 -> 112 there and 325 -> 330 at 64^3.  PF is a template argument: as
+// run-time branches they cost the small applies (50x45x36) 1.4%.
+static const size_t kL2Bytes = (size_t)80 << 20, kSmemSM = 227 * 1024;
+static const int kAhead = 148;
+
+template <typename T, int MODE, bool PF, typename Q, typename Qz>
+static int planes_launch_pf(bdgd_ctx *c, const Prog &p, const FieldsDev &fd, const Q &q, const Qz &qz, const void *x,
                          long long ldx, void *y, long long ldy, void *spec, int nc) {
   typedef typename Cx<T>::t C;
   const size_t sm = sizeof(C) * (size_t)q.rows * q.ld;
   const size_t smz = sizeof(C) * (size_t)q.tx * q.nz;
   int rc;
   if (sm > 48 * 1024) {
-    if ((rc = bdgd_smem_attr(k_plane_fwd<T, MODE, Q>, sm))) return rc;
-    if ((rc = bdgd_smem_attr(k_plane_inv<T, MODE, Q>, sm))) return rc;
+    if ((rc = bdgd_smem_attr(k_plane_fwd<T, MODE, Q, PF>, sm))) return rc;
+    if ((rc = bdgd_smem_attr(k_plane_inv<T, MODE, Q, PF>, sm))) return rc;
   }
   if (smz > 48 * 1024 && (rc = bdgd_smem_attr(k_zlines<T, Qz>, smz))) return rc;
   TwTab<C, Q> ty;
@@ -810,18 +851,29 @@ static int planes_launch(bdgd_ctx *c, const Prog &p, const FieldsDev &fd, const 
   const unsigned nzb = (unsigned)((q.nxk * q.ny + q.tx - 1) / q.tx);
   const int thr = plane_threads<T, Q>();
   C *sp = (C *)spec;
-  if ((rc = launch_after(c, k_plane_fwd<T, MODE, Q>, dim3(nc * p.J, q.nz), thr, sm, c->geo, p, fd, q, ty, x, ldx, sp, y, ldy)))
+  const int ahead = PF && 2 * (sm + 1024) > kSmemSM ? kAhead : 0;
+  if ((rc = launch_after(c, k_plane_fwd<T, MODE, Q, PF>, dim3(nc * p.J, q.nz), thr, sm, c->geo, p, fd, q, ty, x, ldx, sp, y, ldy, ahead)))
     return rc;
   if ((rc = launch_after(c, k_zlines<T, Qz>, dim3(nc * p.J, nzb), kZThreads, smz, c->geo, p, fd, qz, tz, sp,
                          MODE == PL_REAL ? 0.5 : 1.0)))
     return rc;
   const C *csp = sp;
   for (int h = 0; h < p.nh; ++h)
-    if (p.nf[h] > 1 && (rc = launch_after(c, k_plane_inv<T, MODE, Q>, dim3(nc, q.nz), thr, sm, c->geo, p, fd, q, ty, csp, y,
-                                          ldy, h, 1, 1)))
+    if (p.nf[h] > 1 && (rc = launch_after(c, k_plane_inv<T, MODE, Q, PF>, dim3(nc, q.nz), thr, sm, c->geo, p, fd, q, ty, csp, y,
+                                          ldy, h, 1, 1, ahead)))
       return rc;
-  return launch_after(c, k_plane_inv<T, MODE, Q>, dim3(nc * p.nh, q.nz), thr, sm, c->geo, p, fd, q, ty, csp, y, ldy, 0,
-                      p.nh, 0);
+  return launch_after(c, k_plane_inv<T, MODE, Q, PF>, dim3(nc * p.nh, q.nz), thr, sm, c->geo, p, fd, q, ty, csp, y, ldy, 0,
+                      p.nh, 0, ahead);
+}
+
+template <typename T, int MODE, typename Q, typename Qz>
+static int planes_launch(bdgd_ctx *c, const Prog &p, const FieldsDev &fd, const Q &q, const Qz &qz, const void *x,
+                         long long ldx, void *y, long long ldy, void *spec, int nc) {
+  typedef typename Cx<T>::t C;
+  const size_t bytes = (size_t)nc * (2 * p.nh * c->geo.S * (MODE == PL_CPLX ? sizeof(C) : sizeof(T)) +
+                                     p.J * c->geo.H * sizeof(C));
+  if (bytes > kL2Bytes) return planes_launch_pf<T, MODE, true>(c, p, fd, q, qz, x, ldx, y, ldy, spec, nc);
+  return planes_launch_pf<T, MODE, false>(c, p, fd, q, qz, x, ldx, y, ldy, spec, nc);
 }
 
 template <typename T, int MODE>

@@ -58,3 +58,37 @@ def test_planes_match_generic(grid, bdg, monkeypatch):
         got32 = apply(op, 1, x.to(torch.complex64 if cplx else torch.float32), "reg")
         assert float((got32 - ref).abs().max()) < 2e-5 * scale, op
     dc.close()
+
+
+# large applies prefetch into L2 (both plane kernels where a plane fills an SM):
+# the arithmetic is the same, so every column equals that of a one-column apply,
+# which is too small to prefetch, bit for bit
+PREFETCH = [
+    ([128, 128, 128], False, 3, "KM"), ([64, 64, 64], False, 8, "KML"), ([250, 75, 4], False, 70, "KML"),
+    ([256, 60, 4], True, 50, "KML"), ([48, 64, 96], True, 5, "KML"),
+]
+
+
+@pytest.mark.parametrize("case", PREFETCH, ids=lambda c: "x".join(map(str, c[0])) + ("-z" if c[1] else "-d"))
+def test_large_applies_equal_single_columns(case, bdg, monkeypatch):
+    torch = pytest.importorskip("torch")
+    N, cplx, ncol, ops = case
+    monkeypatch.setenv("BDG_FFT_PATH", "reg")
+    rng = np.random.default_rng(8)
+    S = int(np.prod(N))
+    H = S if cplx else (N[0] // 2 + 1) * S // N[0]
+    dc = bdg.DeviceContext(3, N, [0.5 * n for n in N], cplx)
+    wf = rng.standard_normal(S) + (1j * rng.standard_normal(S) if cplx else 0.0)
+    dc.set_fields(ltK=1 + rng.random(S), ltM=2 + rng.random(S), wf=wf, pK=0.5 + rng.random(S), pM=0.5 + rng.random(S),
+                  mu=0.9, vdd=rng.standard_normal(H), g_ddi=0.6, dipolar=True)
+    for o in ops:
+        op, n = {"K": (bdg.OP_K, S), "M": (bdg.OP_M, S), "L": (bdg.OP_LREP, 2 * S)}[o]
+        x = torch.randn((ncol, n), dtype=torch.complex128 if cplx else torch.float64, device="cuda")
+        y, y1 = torch.zeros_like(x), torch.zeros_like(x)
+        torch.cuda.synchronize()
+        dc.apply_ptr(op, 0, x.data_ptr(), n, y.data_ptr(), n, ncol)
+        for j in range(ncol):
+            dc.apply_ptr(op, 0, x[j].data_ptr(), n, y1[j].data_ptr(), n, 1)
+        dc.synchronize()
+        assert float(y.abs().max()) > 0.0 and torch.equal(y, y1), o
+    dc.close()
