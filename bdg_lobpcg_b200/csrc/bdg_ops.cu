@@ -1380,17 +1380,27 @@ static int apply_tuned(bdgd_ctx *c, int op, const Prog &p, int prec, const void 
     float ms[4] = {0.f, 0.f, 0.f, 0.f};
     const bool planes = bdgd_planes_usable(c, prec);
     const int order[3] = {2, planes ? 3 : 1, 1};  // the likely choice last: its result stays in y
+    // A block of many columns is timed on its first nt, still thousands of thread
+    // blocks a launch, between two applies of the whole (the first sizes the
+    // scratch, the second is the result): two whole applies and six partial ones
+    // in place of six whole ones.
+    const long long fill = ((1LL << 23) + c->S - 1) / c->S;
+    const int nt = (int)(fill < 4 ? 4 : fill) < ncol ? (int)(fill < 4 ? 4 : fill) : ncol;
     cudaEvent_t e0, e1;
     BDGD_CK(cudaEventCreate(&e0));
     BDGD_CK(cudaEventCreate(&e1));
     int rc = BDGD_OK;
+    if (nt < ncol) {
+      c->force_path = 1;
+      rc = dispatch(c, p, prec, x, ldx, y, ldy, ncol, 0, 0);
+    }
     for (int i = 0; i < (planes ? 3 : 2) && !rc; ++i) {
       const int k = order[i];
       c->force_path = k;
-      rc = dispatch(c, p, prec, x, ldx, y, ldy, ncol, 0, 0);
+      rc = dispatch(c, p, prec, x, ldx, y, ldy, nt, 0, 0);
       if (!rc) {
         cudaEventRecord(e0, c->stream);
-        rc = dispatch(c, p, prec, x, ldx, y, ldy, ncol, 0, 0);
+        rc = dispatch(c, p, prec, x, ldx, y, ldy, nt, 0, 0);
         cudaEventRecord(e1, c->stream);
         cudaError_t ce = cudaEventSynchronize(e1);
         if (ce != cudaSuccess) rc = bdgd_check(ce, "autotune");
@@ -1406,7 +1416,11 @@ static int apply_tuned(bdgd_ctx *c, int op, const Prog &p, int prec, const void 
     c->tune[op][pi] = reg <= ms[2] ? 1 : 2;
     c->tune_ms[op][pi][0] = reg;
     c->tune_ms[op][pi][1] = ms[2];
-    return BDGD_OK;  // y holds the result of the last run
+    if (nt == ncol) return BDGD_OK;  // y holds the result of the last run
+    c->force_path = c->tune[op][pi] == 1 && c->tune_lines[op][pi] ? 3 : c->tune[op][pi];
+    rc = dispatch(c, p, prec, x, ldx, y, ldy, ncol, 0, 0);
+    c->force_path = 0;
+    return rc;
   }
   if (tunable && c->tune[op][pi]) c->force_path = c->tune[op][pi] == 1 && c->tune_lines[op][pi] ? 3 : c->tune[op][pi];
   const int rc = (c->graphs_on && !bdgd_capturing) ? apply_graph(c, op, p, prec, x, ldx, y, ldy, ncol)
