@@ -203,7 +203,13 @@ constexpr int z_blocks() {
 
 // The kernels are launched programmatically: the blocks of one become resident
 // while the last blocks of the kernel before it run, and wait here for its
-// results (the launch latency of a small apply overlaps).
+// results (the launch latency of a small apply overlaps).  So x, y and the
+// spectra may be written while a kernel that reads them is already resident (x
+// by the inverse of an apply before this one): they are read by ordinary loads,
+// through pointers without __restrict__, after this wait.  The read-only path
+// (__ldg) wants data that no one writes during the kernel's life: the fields and
+// tables, whose uploads end with a wait of the host or a copy, which a launch
+// does not overlap.
 __device__ __forceinline__ void grid_wait() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -231,8 +237,8 @@ template <int THR> __device__ __forceinline__ void prefetch_l2(const void *p, in
 template <typename T, int MODE, typename Q, bool PF>
 __global__ void __launch_bounds__((plane_threads<T, Q>()), (plane_blocks<T, Q>()))
     k_plane_fwd(GeoDev g, Prog p, FieldsDev f, Q q, const __grid_constant__ TwTab<typename Cx<T>::t, Q> tw,
-                const void *__restrict__ xin, long long ldx, typename Cx<T>::t *__restrict__ spec,
-                void *__restrict__ yout, long long ldy, int ahead) {
+                const void *xin, long long ldx, typename Cx<T>::t *spec,
+                void *yout, long long ldy, int ahead) {
   typedef typename Cx<T>::t C;
   extern __shared__ __align__(16) unsigned char smraw[];
   constexpr int THR = plane_threads<T, Q>();
@@ -262,9 +268,9 @@ __global__ void __launch_bounds__((plane_threads<T, Q>()), (plane_blocks<T, Q>()
         const T *sa = (const T *)xin + oc;
         const T *cf = (const T *)pre_coef(f, kind);
 #pragma unroll
-        for (int r = 0; r < R; ++r) v[r].x = __ldg(sa + r * q.x2);
+        for (int r = 0; r < R; ++r) v[r].x = sa[r * q.x2];
 #pragma unroll
-        for (int r = 0; r < R; ++r) v[r].y = __ldg(sa + hs + r * q.x2);
+        for (int r = 0; r < R; ++r) v[r].y = sa[hs + r * q.x2];
         if (local) {
           T *y = (T *)yout + col * ldy + hf * g.S + plane + o;
 #pragma unroll
@@ -300,7 +306,7 @@ __global__ void __launch_bounds__((plane_threads<T, Q>()), (plane_blocks<T, Q>()
         const T *cf = (const T *)pre_coef(f, kind);
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-          v[r].x = __ldg(src + r * q.x2);
+          v[r].x = src[r * q.x2];
           v[r].y = cf ? __ldg(cf + plane + o + r * q.x2) : (T)0;
         }
         if (local) {
@@ -315,7 +321,7 @@ __global__ void __launch_bounds__((plane_threads<T, Q>()), (plane_blocks<T, Q>()
         const T *cr = (kind == PRE_PK || kind == PRE_PM) ? (const T *)pre_coef(f, kind) : nullptr;
         const C *cw = (kind == PRE_CONJWF || kind == PRE_DENS) ? (const C *)f.w : nullptr;
 #pragma unroll
-        for (int r = 0; r < R; ++r) v[r] = __ldg(src + r * q.x2);
+        for (int r = 0; r < R; ++r) v[r] = src[r * q.x2];
         if (local) {
           C *y = (C *)yout + col * ldy + hf * g.S + plane + o;
           T c[R];
@@ -464,7 +470,7 @@ __global__ void __launch_bounds__((plane_threads<T, Q>()), (plane_blocks<T, Q>()
 // ---------------------------------------------------------------------------
 template <typename T, typename Q>
 __global__ void __launch_bounds__(kZThreads, (z_blocks<T, Q>()))
-    k_zlines(GeoDev g, Prog p, FieldsDev f, Q q, const __grid_constant__ TwTab<typename Cx<T>::t, Q> tw, typename Cx<T>::t *__restrict__ spec, double sc) {
+    k_zlines(GeoDev g, Prog p, FieldsDev f, Q q, const __grid_constant__ TwTab<typename Cx<T>::t, Q> tw, typename Cx<T>::t *spec, double sc) {
   typedef typename Cx<T>::t C;
   extern __shared__ __align__(16) unsigned char smraw[];
   C *P = (C *)smraw;
@@ -559,7 +565,7 @@ __global__ void __launch_bounds__(kZThreads, (z_blocks<T, Q>()))
 template <typename T, int MODE, typename Q, bool PF>
 __global__ void __launch_bounds__((plane_threads<T, Q>()), (plane_blocks<T, Q>()))
     k_plane_inv(GeoDev g, Prog p, FieldsDev f, Q q, const __grid_constant__ TwTab<typename Cx<T>::t, Q> tw,
-                const typename Cx<T>::t *__restrict__ spec, void *yout, long long ldy, int h0, int nhs, int fi, int ahead) {
+                const typename Cx<T>::t *spec, void *yout, long long ldy, int h0, int nhs, int fi, int ahead) {
   typedef typename Cx<T>::t C;
   extern __shared__ __align__(16) unsigned char smraw[];
   constexpr int THR = plane_threads<T, Q>();
@@ -583,7 +589,7 @@ __global__ void __launch_bounds__((plane_threads<T, Q>()), (plane_blocks<T, Q>()
       const int t = fdiv(i, q.dnxk), k = i - t * q.nxk;
       C v[R];
 #pragma unroll
-      for (int r = 0; r < R; ++r) v[r] = __ldg(in + (q.ye * r + t) * q.nxk + k);
+      for (int r = 0; r < R; ++r) v[r] = in[(q.ye * r + t) * q.nxk + k];
       rdft<R, +1>(v);
       twiddle_c<R, +1>(v, tw, t);
       const bool up = MODE == PL_REAL && 2 * t >= q.ye;
