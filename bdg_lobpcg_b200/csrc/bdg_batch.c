@@ -10,8 +10,9 @@
  * work and small kernels of the others.  Operator applies are replayed as
  * CUDA graphs when `graphs` is set, and the FFT pass family of every
  * context is chosen by the library's autotuner (bdgd_fft_tuning).  After each
- * solve the problem's solver workspace and scratch are released, so device
- * memory holds at most `concurrency` workspaces.
+ * solve the problem's solver workspace and scratch are released and its library
+ * handles pass to the next problem of the thread, so device memory holds at
+ * most `concurrency` workspaces and sets of handles.
  */
 #include <pthread.h>
 #include <stdio.h>
@@ -26,6 +27,10 @@
 
 void bdg_solver_release(bdg_t *bdg);
 void bdg_solver_release_memory(bdg_t *bdg);
+void *bdg_handles_new(void);
+void bdg_handles_lend(void *handles, bdg_t *bdg);
+void bdg_handles_return(void *handles, bdg_t *bdg);
+void bdg_handles_free(void *handles);
 
 typedef struct {
   bdg_t **p;
@@ -34,6 +39,8 @@ typedef struct {
   int graphs;
   int *rcs;
   double *secs;
+  void **handles; /* of the workers, nhandles of them */
+  int nhandles;
   pthread_mutex_t mu;
 } batch_t;
 
@@ -51,6 +58,10 @@ void bdg_release_device_memory(bdg_t *bdg) {
 
 static void *batch_worker(void *arg) {
   batch_t *b = (batch_t *)arg;
+  void *handles = bdg_handles_new();
+  pthread_mutex_lock(&b->mu);
+  b->handles[b->nhandles++] = handles;
+  pthread_mutex_unlock(&b->mu);
   for (;;) {
     pthread_mutex_lock(&b->mu);
     const int i = b->next++;
@@ -63,11 +74,13 @@ static void *batch_worker(void *arg) {
       bdgd_ctx *d = bdg_device_context(p);
       if (d) bdgd_set_graphs(d, 1);
     }
+    bdg_handles_lend(handles, p);
     rc = bdg_solve(p);
     if (b->secs) b->secs[i] = wall() - t0;
     if (b->rcs) b->rcs[i] = rc;
-    /* the library handles stay until every worker has ended (see ws_free) */
+    /* no handle is destroyed before every worker has ended (see ws_free) */
     bdg_solver_release_memory(p);
+    bdg_handles_return(handles, p);
     if (p->ctx && p->ctx->dev) bdgd_trim(p->ctx->dev);
   }
   return NULL;
@@ -85,6 +98,7 @@ int bdg_solve_batch(bdg_t **problems, int n, int concurrency, int graphs, int *r
   b.graphs = graphs;
   b.rcs = rcs_out ? rcs_out : (int *)calloc((size_t)n, sizeof(int));
   b.secs = seconds_out;
+  b.handles = (void **)calloc((size_t)concurrency, sizeof(void *));
   pthread_mutex_init(&b.mu, NULL);
   pthread_t *th = (pthread_t *)calloc((size_t)concurrency, sizeof(pthread_t));
   int started = 0; /* handles of the threads created, stored contiguously */
@@ -93,6 +107,8 @@ int bdg_solve_batch(bdg_t **problems, int n, int concurrency, int graphs, int *r
   if (started == 0) batch_worker(&b); /* no threads available: solve here */
   for (int t = 0; t < started; ++t) pthread_join(th[t], NULL);
   free(th);
+  for (int i = 0; i < b.nhandles; ++i) bdg_handles_free(b.handles[i]);
+  free(b.handles);
   for (int i = 0; i < n; ++i) bdg_solver_release(problems[i]);
   pthread_mutex_destroy(&b.mu);
   int bad = 0;

@@ -119,8 +119,8 @@ static void dfree(ws_t *w, void *p) {
 
 /* Free the workspace; its library handles only with `handles`.  Destroying them
  * synchronises the device, and the driver crashed in that call (now and then,
- * inside cuCtxSynchronize) while other threads' solves were running, so the
- * workers of bdg_solve_batch leave them to the thread that joins them. */
+ * inside cuCtxSynchronize) while other threads' solves were running, so
+ * bdg_solve_batch destroys them after its workers have ended. */
 static void ws_free(ws_t *w, int handles) {
   if (!w) return;
   for (int i = 0; i < NB_COUNT; i++)
@@ -254,6 +254,61 @@ void bdg_solver_release_memory(bdg_t *bdg) {
     ws_free(&((ws_t *)bdg->solver_ws)[1], 0);
   }
   safe_free(&bdg->block);
+}
+
+/* Library handles of a worker of bdg_solve_batch, one pair for each workspace.
+ * The worker lends them to the problem that it solves: a pair holds 350 MB of
+ * device memory, so with a pair for each problem the memory of a batch grew with
+ * its length (48 problems of 16^3, two at a time: 17 GB). */
+typedef struct {
+  cublasHandle_t blas[2];
+  cusolverDnHandle_t sol[2];
+} handles_t;
+
+void *bdg_handles_new(void) { return xcalloc(1, sizeof(handles_t)); }
+
+/* to the workspaces that have none */
+void bdg_handles_lend(void *handles, bdg_t *bdg) {
+  handles_t *h = (handles_t *)handles;
+  if (!bdg->solver_ws) bdg->solver_ws = xcalloc(2, sizeof(ws_t));
+  for (int i = 0; i < 2; i++) {
+    ws_t *w = &((ws_t *)bdg->solver_ws)[i];
+    if (!w->blas) {
+      w->blas = h->blas[i];
+      h->blas[i] = NULL;
+    }
+    if (!w->sol) {
+      w->sol = h->sol[i];
+      h->sol[i] = NULL;
+    }
+  }
+}
+
+/* back, with those that the solve created, after the work queued with them; a
+ * problem that had handles of its own keeps those that find no place */
+void bdg_handles_return(void *handles, bdg_t *bdg) {
+  handles_t *h = (handles_t *)handles;
+  if (bdg->ctx && bdg->ctx->dev) bdgd_synchronize(bdg->ctx->dev);
+  for (int i = 0; i < 2; i++) {
+    ws_t *w = &((ws_t *)bdg->solver_ws)[i];
+    if (!h->blas[i]) {
+      h->blas[i] = w->blas;
+      w->blas = NULL;
+    }
+    if (!h->sol[i]) {
+      h->sol[i] = w->sol;
+      w->sol = NULL;
+    }
+  }
+}
+
+void bdg_handles_free(void *handles) {
+  handles_t *h = (handles_t *)handles;
+  for (int i = 0; i < 2; i++) {
+    if (h->blas[i]) cublasDestroy(h->blas[i]);
+    if (h->sol[i]) cusolverDnDestroy(h->sol[i]);
+  }
+  free(h);
 }
 
 void bdg_solver_release(bdg_t *bdg) {
