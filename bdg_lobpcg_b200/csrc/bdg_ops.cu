@@ -1036,20 +1036,21 @@ static int cols_ct(bdgd_ctx *c, const Prog &p, const FieldsDev &fd, typename Cx<
   return BDGD_ERR_UNSUPPORTED;
 }
 
-// FFT pass family: register transforms (default; the plane passes where they
-// can run, else the line passes), compile-time sized shared-memory stages, or
-// the generic runtime-sized kernels.  BDG_FFT_PATH = reg | lines | ct | generic
-// overrides (BDG_GENERIC_FFT=1 is the same as generic).
-enum { FFT_PATH_REG = 0, FFT_PATH_CT = 1, FFT_PATH_GENERIC = 2, FFT_PATH_LINES = 3 };
+// FFT pass family: register transforms (the plane passes where they can run,
+// else the line passes), compile-time sized shared-memory stages, or the generic
+// runtime-sized kernels.  Without a choice (FFT_PATH_AUTO) register transforms,
+// their form for few columns by bdgd_planes_pay().  BDG_FFT_PATH = reg | lines |
+// ct | generic overrides (BDG_GENERIC_FFT=1 is the same as generic).
+enum { FFT_PATH_REG = 0, FFT_PATH_CT = 1, FFT_PATH_GENERIC = 2, FFT_PATH_LINES = 3, FFT_PATH_AUTO = 4 };
+static const int kTuneCols = 4;  // applies of fewer columns are not timed
 static int fft_path(const bdgd_ctx *c) {
   if (c->force_path) return c->force_path == 2 ? FFT_PATH_CT : c->force_path == 3 ? FFT_PATH_LINES : FFT_PATH_REG;
   if (getenv("BDG_GENERIC_FFT")) return FFT_PATH_GENERIC;
   const char *e = getenv("BDG_FFT_PATH");
-  if (e) {
-    if (!strcmp(e, "lines")) return FFT_PATH_LINES;
-    if (!strcmp(e, "ct")) return FFT_PATH_CT;
-    if (!strcmp(e, "generic")) return FFT_PATH_GENERIC;
-  }
+  if (!e) return FFT_PATH_AUTO;
+  if (!strcmp(e, "lines")) return FFT_PATH_LINES;
+  if (!strcmp(e, "ct")) return FFT_PATH_CT;
+  if (!strcmp(e, "generic")) return FFT_PATH_GENERIC;
   return FFT_PATH_REG;
 }
 
@@ -1087,8 +1088,12 @@ static int run_program(bdgd_ctx *c, const Prog &p, const void *x, long long ldx,
   }
   // column chunking bounded by the scratch cap
   const size_t per_col = sizeof(C) * (size_t)p.J * (size_t)g.H;
-  const bool planes = !only_fwd && !only_bwd && fft_path(c) == FFT_PATH_REG &&
-                      bdgd_planes_usable(c, f32 ? BDGD_F32 : BDGD_F64);
+  const int path = fft_path(c), prec = f32 ? BDGD_F32 : BDGD_F64;
+  const bool lines = !only_fwd && !only_bwd && (path == FFT_PATH_REG || path == FFT_PATH_LINES || path == FFT_PATH_AUTO) &&
+                     bdgd_lines_usable(c, p);
+  const bool planes = !only_fwd && !only_bwd && (path == FFT_PATH_REG || path == FFT_PATH_AUTO) &&
+                      bdgd_planes_usable(c, prec) &&
+                      !(path == FFT_PATH_AUTO && ncol < kTuneCols && lines && !bdgd_planes_pay(c, p, prec, ncol));
   int chunk = ncol;
   if (per_col * (size_t)chunk > c->spec_cap) {
     chunk = (int)(c->spec_cap / per_col);
@@ -1113,7 +1118,7 @@ static int run_program(bdgd_ctx *c, const Prog &p, const void *x, long long ldx,
     }
     return BDGD_OK;
   }
-  if (!only_fwd && !only_bwd && (fft_path(c) == FFT_PATH_REG || fft_path(c) == FFT_PATH_LINES) && bdgd_lines_usable(c, p)) {
+  if (lines) {
     for (int c0 = 0; c0 < ncol; c0 += chunk) {
       const int nc = (ncol - c0) < chunk ? (ncol - c0) : chunk;
       const size_t esz = CPLX ? sizeof(C) : sizeof(T);
@@ -1125,7 +1130,7 @@ static int run_program(bdgd_ctx *c, const Prog &p, const void *x, long long ldx,
     return BDGD_OK;
   }
   const bool ct = (c->dim >= 2) && ct_supported(c->N[0]) && ct_supported(c->N[1]) &&
-                  (c->dim < 3 || ct_supported(c->N[2])) && fft_path(c) != FFT_PATH_GENERIC;
+                  (c->dim < 3 || ct_supported(c->N[2])) && path != FFT_PATH_GENERIC;
   if (ct) {
     for (int c0 = 0; c0 < ncol; c0 += chunk) {
       const int nc = (ncol - c0) < chunk ? (ncol - c0) : chunk;
@@ -1375,7 +1380,7 @@ static int apply_tuned(bdgd_ctx *c, int op, const Prog &p, int prec, const void 
   const int pi = prec == BDGD_F32 ? 1 : 0;
   const bool env = getenv("BDG_FFT_PATH") || getenv("BDG_GENERIC_FFT");
   const bool tunable = !env && bdgd_lines_usable(c, p) && op < 16;
-  if (tunable && c->tune[op][pi] == 0 && ncol >= 4 && !bdgd_capturing) {
+  if (tunable && c->tune[op][pi] == 0 && ncol >= kTuneCols && !bdgd_capturing) {
     // force_path: 1 plane passes, 2 shared-memory stages, 3 line passes
     float ms[4] = {0.f, 0.f, 0.f, 0.f};
     const bool planes = bdgd_planes_usable(c, prec);
@@ -1423,6 +1428,7 @@ static int apply_tuned(bdgd_ctx *c, int op, const Prog &p, int prec, const void 
     return rc;
   }
   if (tunable && c->tune[op][pi]) c->force_path = c->tune[op][pi] == 1 && c->tune_lines[op][pi] ? 3 : c->tune[op][pi];
+  if (c->force_path == 1 && ncol < kTuneCols) c->force_path = 0;  // planes won for more columns than these
   const int rc = (c->graphs_on && !bdgd_capturing) ? apply_graph(c, op, p, prec, x, ldx, y, ldy, ncol)
                                                    : dispatch(c, p, prec, x, ldx, y, ldy, ncol, 0, 0);
   c->force_path = 0;

@@ -11,6 +11,10 @@
 // fits one block's shared memory.
 bool bdgd_planes_usable(const bdgd_ctx *c, int prec);
 
+// Whether an apply of few columns is better done by plane passes than by line
+// passes, on a context where both can run.
+bool bdgd_planes_pay(const bdgd_ctx *c, const Prog &p, int prec, int nc);
+
 // Full operator apply of program p on nc columns; spec holds nc * p.J spectra.
 int bdgd_planes_apply_f64(bdgd_ctx *c, const Prog &p, const FieldsDev &fd, const void *x, long long ldx, void *y,
                           long long ldy, void *spec, int nc);
