@@ -796,8 +796,8 @@ static int rayleigh_ritz(ws_t *w, bdgd_ctx *dev, int k, int m, double drop, doub
   if (chol) {
     /* A_s is well conditioned nearly always: with Z^T A_s Z = I the pencil is
      * H = Z^T B_s Z alone, one eigen-decomposition in place of three.  The
-     * smallest pivot comes back with the eigenvalues. */
-    double piv = 0.0;
+     * smallest pivot comes back with the eigenvalues and is looked at before
+     * them: those of a rejected factor say nothing. */
     TRY(zgemm_small(w, 0, 0, k, k, k, 1.0, w->Gb, k, w->Z, k, 0.0, w->T1s, k));
     TRY(zgemm_small(w, 1, 0, k, k, k, 1.0, w->Z, k, w->T1s, k, 0.0, w->Ya, k));
     DEV_TRY(bdgd_hermitize(dev, w->Ya, k, cplx));
@@ -808,22 +808,21 @@ static int rayleigh_ritz(ws_t *w, bdgd_ctx *dev, int k, int m, double drop, doub
     TRY(eig_top_launch(w, dev, w->Ya, k, m, &own));
     double chk[3] = {0.0, 0.0, 0.0};
     CUDA_TRY(cudaMemcpyAsync(chk, w->piv, sizeof chk, cudaMemcpyDeviceToHost, stream_of(dev)));
-    if (own) TRY(host_vec(w, dev, w->wH, k, h));
-    if (own && !(chk[1] >= EIG_PIV && chk[2] <= EIG_RES)) own = 0; /* H is untouched */
-    if (own) {
+    TRY(host_vec(w, dev, w->wH, own ? k : 1, h));
+    chol = chol_good(w, chk[0]);
+    if (chol && own && chk[1] >= EIG_PIV && chk[2] <= EIG_RES) {
       Q = w->V;
       th = w->wH + (k - m);
       nq = m;
-    } else {
+    } else if (chol) { /* H is untouched */
       TRY(heev(w, w->Ya, k, k, w->wH));
       TRY(host_vec(w, dev, w->wH, k, h));
     }
-    piv = chk[0];
     /* the rounding of H is relative to its largest value: with an undeflated
      * zero mode (theta = 1/lambda large) the other values would carry it, so
      * the graded eigen-decompositions below serve for the rest of the solve */
-    if (k >= m && h[k - 1] > THETA_SPREAD * fabs(h[k - m])) w->graded = 1;
-    if (chol_good(w, piv) && !w->graded) {
+    if (chol && k >= m && h[k - 1] > THETA_SPREAD * fabs(h[k - m])) w->graded = 1;
+    if (chol && !w->graded) {
       int npos = 0;
       for (int i = 0; i < k; i++)
         if (h[i] > 0) npos++;
