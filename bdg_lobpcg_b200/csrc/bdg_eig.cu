@@ -20,7 +20,9 @@
 // cluster the random starts give independent combinations.  Orthonormalising
 // mixes vectors by their overlaps, which leaves the residuals as they are.  The
 // caller checks the residuals (d_check) and the smallest pivot of the Gram
-// matrix and falls back to syevd.
+// matrix and falls back to syevd.  The residuals are those of the tridiagonal
+// matrix, so a matrix whose squares leave the range of a double would pass the
+// check with a wrong reduction: k_tridiag scales by a power of two.
 #include <cuda_runtime.h>
 #include <math.h>
 
@@ -89,23 +91,46 @@ __device__ __forceinline__ double warp_sum(double s) {
 // registers a thread would spill the matrix, and the sixteenth does both
 template <int NB> constexpr int tri_threads() { return EIG_THREADS + (NB <= 3 ? 32 : 0); }
 
+// exponent of the largest element by its high word, 0 where that needs no scaling
+__device__ __forceinline__ int tri_scale(unsigned top) {
+  const int ex = (int)(top >> 20) - 1023;
+  return (ex > 256 || ex < -256) && ex < 1024 && top != 0 ? ex : 0;
+}
+
 template <int NB>
 __global__ void __launch_bounds__(tri_threads<NB>()) k_tridiag(const double *__restrict__ A, int k, double *__restrict__ V,
                                                               double *__restrict__ tau, double *__restrict__ d,
                                                               double *__restrict__ e) {
   constexpr int K = 32 * NB, NR = 2 * NB, NF = NR <= 2 ? 2 : NR <= 4 ? 4 : NR <= 8 ? 8 : 16;
   __shared__ double xs[2][K], ys[2][K], ps[K], pf[K], vs[K], part[16][K], red[NB], par[2];
+  __shared__ unsigned top;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  if (threadIdx.x == 0) top = 0;
   double a[NR][NB];
+  unsigned big = 0;  // largest high word without its sign: the exponent, in order of magnitude
 #pragma unroll
   for (int r = 0; r < NR; ++r)
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
       const int i = 16 * r + ty, c = 32 * b + tx;
       a[r][b] = (ty < 16 && i < k && c <= i) ? A[(long long)c * k + i] : 0.0;
+      big = max(big, (unsigned)__double2hiint(a[r][b]) & 0x7fffffffu);
     }
   for (int i = threadIdx.x; i < K; i += tri_threads<NB>()) xs[0][i] = xs[1][i] = ys[0][i] = ys[1][i] = ps[i] = pf[i] = vs[i] = 0.0;
   __syncthreads();
+  big = __reduce_max_sync(0xffffffffu, big);
+  if (tx == 0) atomicMax(&top, big);
+  __syncthreads();
+  // far from one: the largest element to [1, 2), d and e scaled back at the end
+  // (by two factors, as 2^ex may leave the range).  Infinities and NaN stay
+  if (const int ex = tri_scale(top)) {
+    const int e1 = ex / 2, e2 = ex - e1;
+    const double f1 = __hiloint2double((1023 - e1) << 20, 0), f2 = __hiloint2double((1023 - e2) << 20, 0);
+#pragma unroll
+    for (int r = 0; r < NR; ++r)
+#pragma unroll
+      for (int b = 0; b < NB; ++b) a[r][b] = a[r][b] * f1 * f2;
+  }
   for (int j = 0; j < k - 2; ++j) {
     double *x = xs[j & 1], *y = ys[j & 1];
     if (ty < 16) {
@@ -235,6 +260,15 @@ __global__ void __launch_bounds__(tri_threads<NB>()) k_tridiag(const double *__r
         if (i == k - 1 && c == k - 2) e[c] = a[r][b];
       }
     }
+  if (const int ex = tri_scale(top)) {
+    __syncthreads();
+    const int e1 = ex / 2, e2 = ex - e1;
+    const double f1 = __hiloint2double((1023 + e1) << 20, 0), f2 = __hiloint2double((1023 + e2) << 20, 0);
+    for (int i = threadIdx.x; i < k; i += tri_threads<NB>()) {
+      d[i] = d[i] * f1 * f2;
+      if (i + 1 < k) e[i] = e[i] * f1 * f2;
+    }
+  }
 }
 
 // Gershgorin bounds of the tridiagonal matrix, by one warp
