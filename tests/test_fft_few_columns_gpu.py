@@ -4,7 +4,7 @@ The autotuner times applies of four columns or more.  Below, plane passes serve
 the grids where they pay and line passes the others, by a rule on sizes, precision
 and operator.  An apply that nothing chooses equals, bit for bit, the one of the
 family that the rule names, and launches as many kernels (planes 3, or 4 with a
-half of two fields; lines 5); the two families agree to 1e-12 (FP64) and 2e-5
+half of two fields; lines 3 and two for each half); the two families agree to 1e-12 (FP64) and 2e-5
 (FP32) of the largest entry.  Also where a block was tuned before: the tuner's
 choice of planes is one for many columns.
 """
