@@ -391,12 +391,7 @@ __device__ __forceinline__ void gram_tile_rows(const GTask &tk, int ti, int tj, 
   typedef typename GStageV<T, CPLX, V>::E E;
   constexpr int RK = GStageV<T, CPLX, V>::RK, LDE = GStageV<T, CPLX, V>::LDE;
   constexpr int ES = CPLX ? 2 : 1;
-  // SPLIT (complex, V = 2, 256 threads): warps 0-3 accumulate the real parts
-  // and warps 4-7 the imaginary parts of the same four 32 x 32 quadrants, one
-  // accumulator set per warp
-  constexpr bool SPLIT = CPLX && V == 2;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int part = SPLIT ? (warp >> 2) : 0;
   const int wi = warp & 1, wj = (warp >> 1) & 1;
   const int lr = lane & 3, lc = lane >> 2;
   double acc[4][4][2], aci[4][4][2];
@@ -471,39 +466,19 @@ __device__ __forceinline__ void gram_tile_rows(const GTask &tk, int ti, int tj, 
         br[nj] = re_of<E>(v);
         bi[nj] = im_of<E>(v);
       }
-      if constexpr (SPLIT) {
-        if (part == 0) {
 #pragma unroll
-          for (int mi = 0; mi < 4; ++mi)
+      for (int mi = 0; mi < 4; ++mi)
 #pragma unroll
-            for (int nj = 0; nj < 4; ++nj) {
-              dmma(acc[mi][nj][0], acc[mi][nj][1], ar[mi], br[nj]);
-              dmma(acc[mi][nj][0], acc[mi][nj][1], ai[mi], bi[nj]);
-            }
-        } else {
-#pragma unroll
-          for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-            for (int nj = 0; nj < 4; ++nj) {
-              dmma(acc[mi][nj][0], acc[mi][nj][1], ar[mi], bi[nj]);
-              dmma(acc[mi][nj][0], acc[mi][nj][1], -ai[mi], br[nj]);
-            }
-        }
-      } else {
+        for (int nj = 0; nj < 4; ++nj) dmma(acc[mi][nj][0], acc[mi][nj][1], ar[mi], br[nj]);
+      if (CPLX) {
 #pragma unroll
         for (int mi = 0; mi < 4; ++mi)
 #pragma unroll
-          for (int nj = 0; nj < 4; ++nj) dmma(acc[mi][nj][0], acc[mi][nj][1], ar[mi], br[nj]);
-        if (CPLX) {
-#pragma unroll
-          for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-            for (int nj = 0; nj < 4; ++nj) {
-              dmma(acc[mi][nj][0], acc[mi][nj][1], ai[mi], bi[nj]);
-              dmma(aci[mi][nj][0], aci[mi][nj][1], ar[mi], bi[nj]);
-              dmma(aci[mi][nj][0], aci[mi][nj][1], -ai[mi], br[nj]);
-            }
-        }
+          for (int nj = 0; nj < 4; ++nj) {
+            dmma(acc[mi][nj][0], acc[mi][nj][1], ai[mi], bi[nj]);
+            dmma(aci[mi][nj][0], aci[mi][nj][1], ar[mi], bi[nj]);
+            dmma(aci[mi][nj][0], aci[mi][nj][1], -ai[mi], br[nj]);
+          }
       }
     }
     if constexpr (NS == 2) __syncthreads();
@@ -522,12 +497,8 @@ __device__ __forceinline__ void gram_tile_rows(const GTask &tk, int ti, int tj, 
         const int il = wi * 32 + mi * 8 + lc;
         const int jl = wj * 32 + nj * 8 + 2 * lr + e;
         const long long o = ((long long)jl * GT + il) * ES;
-        if constexpr (SPLIT) {
-          out[o + part] = acc[mi][nj][e];
-        } else {
-          out[o] = acc[mi][nj][e];
-          if (CPLX) out[o + 1] = aci[mi][nj][e];
-        }
+        out[o] = acc[mi][nj][e];
+        if (CPLX) out[o + 1] = aci[mi][nj][e];
       }
 }
 

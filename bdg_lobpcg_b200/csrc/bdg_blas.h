@@ -42,9 +42,9 @@ int bdgd_chol_inverse(bdgd_ctx *c, const double *G, int k, int ldg, double *Z, d
 /* All eigenvalues (w, ascending) of the symmetric A (k x k, column-major, not
  * changed) and unit eigenvectors Y (k x nv) of the nv largest, those of close
  * eigenvalues not orthogonal to each other (bdg_eig.cu); *d_check the largest
- * residual relative to ||A||.  work: bdgd_eig_work(k, nv) bytes.  3 <= k <= 192,
+ * residual relative to ||A||.  work: bdgd_eig_work(k) bytes.  3 <= k <= 192,
  * else BDGD_ERR_UNSUPPORTED. */
-size_t bdgd_eig_work(int k, int nv);
+size_t bdgd_eig_work(int k);
 int bdgd_eig_top(bdgd_ctx *c, const double *A, int k, int nv, double *w, double *Y, double *work, double *d_check);
 int bdgd_hermitize(bdgd_ctx *c, double *A, int k, int cplx);
 int bdgd_clamp(bdgd_ctx *c, double *w, int n, double floor_rel);

@@ -521,9 +521,8 @@ __global__ void __launch_bounds__(32) k_backtr(const double *__restrict__ V, con
   }
 }
 
-extern "C" size_t bdgd_eig_work(int k, int nv) {
+extern "C" size_t bdgd_eig_work(int k) {
   // V, tau, d, e
-  (void)nv;
   return sizeof(double) * ((size_t)k * k + 3 * (size_t)k);
 }
 

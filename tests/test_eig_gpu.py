@@ -53,14 +53,14 @@ class _Eig:
         self.torch = torch
         self.f, self.work = bdg.lib().bdgd_eig_top, bdg.lib().bdgd_eig_work
         self.f.restype, self.f.argtypes = C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_int] + [C.c_void_p] * 4
-        self.work.restype, self.work.argtypes = C.c_size_t, [C.c_int, C.c_int]
+        self.work.restype, self.work.argtypes = C.c_size_t, [C.c_int]
         self.dc = bdg.DeviceContext(1, [16], [1.0], False)
 
     def __call__(self, A, nv):
         torch, k = self.torch, A.shape[0]
         new = lambda *s: torch.full(s, 7.0, dtype=torch.float64, device="cuda")
         a, w, y, chk = torch.tensor(A).cuda(), new(k), new(max(nv, 1), k), new(1)
-        work = new(self.work(k, nv) // 8)
+        work = new(self.work(k) // 8)
         torch.cuda.synchronize()
         rc = self.f(self.dc.ptr, a.data_ptr(), k, nv, w.data_ptr(), y.data_ptr(), work.data_ptr(), chk.data_ptr())
         self.dc.synchronize()
