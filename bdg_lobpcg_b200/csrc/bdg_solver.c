@@ -479,7 +479,7 @@ static int ws_setup(ws_t *w, bdgd_ctx *dev, uint64_t S, uint64_t m, uint64_t nev
   TRY(dmalloc(w, (void **)&w->piv, 4 * sizeof(double)));
   if (!cplx) {
     const int ke = w->K < BDGD_CHOL_MAX ? w->K : BDGD_CHOL_MAX;
-    TRY(dmalloc(w, (void **)&w->eigw, bdgd_eig_work(ke, (int)m < ke ? (int)m : ke)));
+    TRY(dmalloc(w, (void **)&w->eigw, bdgd_eig_work(ke)));
   }
   TRY(dmalloc(w, (void **)&w->colmap, (size_t)w->K * sizeof(int)));
   TRY(dmalloc(w, (void **)&w->actcols, (size_t)w->K * sizeof(int)));
@@ -1273,9 +1273,10 @@ static int run_loop(ws_t *w, bdgd_ctx *dev, bdg_t *bdg, const loop_opts_t *o, do
         swapb(w, NB_P, NB_T1);
         swapb(w, NB_AP, NB_T2);
       } else {
-        /* the projected P enters [X, P] as it is: the W projection's
-         * pseudo-inverse and the Rayleigh-Ritz step's scaled eigen-
-         * decomposition drop its dependent directions */
+        /* the projected P enters [X, P] as it is: where its directions are
+         * dependent, the pivots of the W projection and of the Rayleigh-Ritz
+         * step reject their Cholesky factors, and the eigen-decompositions
+         * that take over drop them */
         pk = p;
       }
     }
