@@ -6,7 +6,11 @@
 // FFTW (src/kinetic_impl.inc:17-30, src/matmulK_impl.inc:11-28,
 // src/matmulM_impl.inc:14-44, src/dipolar_conv_impl.inc:22-52,
 // src/precond_impl.inc:21-118).  Here one launch per FFT pass handles all
-// columns (and both halves [u; v]) of a block:
+// columns (and both halves [u; v]) of a block.  Most 3D applies run in the three
+// plane passes of bdg_planes.cuh, others in the line passes of bdg_lines.cu; this
+// file chooses between them (fft_path, apply_tuned) and holds the two families
+// that stage lines in shared memory, with compile-time and with run-time sizes
+// (all grids, 1D and the raw transforms too):
 //
 //   pass X-fwd   rows along x: prologue (p*x, conj(psi0)*x) + forward FFT
 //   pass Y-fwd   pencils along y (3D only)
@@ -16,10 +20,10 @@
 //   pass X-inv   rows: inverse FFT of every spectrum of the half + epilogue
 //                (+ localTerm*x, + 2 g psi0 * exchange, * p)
 //
-// Each pass stages its lines in shared memory and runs a mixed-radix
-// Stockham FFT (radix 8/4/2/3 butterflies in registers, generic radix for
-// other small primes).  Real fields use the r2c half spectrum (x extent
-// N/2+1) between passes, so the spectrum traffic is that of FFTW's r2c.
+// Each of these passes runs a mixed-radix Stockham FFT (radix 8/4/2/3 butterflies
+// in registers, generic radix for other small primes).  Real fields use the r2c
+// half spectrum (x extent N/2+1) between passes, so the spectrum traffic is that
+// of FFTW's r2c.
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -881,8 +885,7 @@ static int build_ptab(bdgd_ctx *c) {
   return upload_done(c);
 }
 
-// upload a host double array and its float copy
-// FP64 array and its FP32 copy, which the device rounds itself: rounding on the
+// Upload a host FP64 array; its FP32 copy the device rounds itself: rounding on the
 // host and a second copy took longer than the first.  No wait: upload_done().
 static int upload_pair(bdgd_ctx *c, double **d64, float **d32, const double *h, long long n) {
   if (!*d64) BDGD_CK(cudaMalloc((void **)d64, sizeof(double) * n));

@@ -41,9 +41,9 @@
 // item a thread; 128 registers and two blocks took 121 + 227 us for the two
 // plane kernels against 119 + 128).  128^3 FP64 planes take 139 KB, one block an
 // SM.  Whole applies, line passes before against plane passes: Lrep 64^3 FP64, 32
-// columns 464 -> 337 us; T 128^3 FP64, 64 columns 4954 -> 3624 us; Lrep 128^3
-// FP32, 64 columns 4463 -> 2929 us; M 48^3, one column 30 -> 25 us; 50x45x36 FP64
-// (run-time sized stages before), 16 columns 597 -> 108 us.  Chunks of columns
+// columns 459 -> 320 us; T 128^3 FP64, 64 columns 4849 -> 3556 us; Lrep 128^3
+// FP32, 64 columns 4448 -> 2800 us; M 48^3, one column 30 -> 25 us; 50x45x36 FP64
+// (run-time sized stages before), 16 columns 599 -> 110 us.  Chunks of columns
 // whose spectra stay in L2 were slower at every size (64^3: 360 us at 120 MB):
 // the last waves of the many small launches cost more than DRAM does.
 //
@@ -828,9 +828,9 @@ static int launch_after(bdgd_ctx *c, K kern, dim3 grid, int threads, size_t sm, 
 // one plane fills an SM (128^3 FP64: 139 KB) nothing else hides the loads, so
 // both plane kernels also ask for the plane of the block kAhead = 148 SMs
 // later.  Without -> with: Lrep 48x64x96
-// complex 667 -> 640 us; T 128^3 FP64, 64 columns 3666 -> 3549 (the inverse's
-// lookahead alone 3560); Lrep 64^3 FP64, 32 columns 337.4 -> 335.3; Lrep 128^3
-// FP32 unchanged.  Elsewhere they cost: y below kL2Bytes 106.6 -> 107.4
+// complex 667 -> 651 us; T 128^3 FP64, 64 columns 3659 -> 3552 (the inverse's
+// lookahead alone gave nearly all of it); Lrep 64^3 FP64, 32 columns 333.8 ->
+// 331.8; Lrep 128^3 FP32, 64 columns 2901 -> 2882.  Elsewhere they cost: y below kL2Bytes 106.6 -> 107.4
 // (50x45x36, 16 columns), lookahead of both with two or more blocks an SM
 // 106.6 -> 112 there and 325 -> 330 at 64^3.  PF is a template argument: as
 // run-time branches they cost the small applies (50x45x36) 1.4%.
@@ -903,6 +903,10 @@ static int planes_apply(bdgd_ctx *c, const Prog &p, const FieldsDev &fd, const v
   if (!bdgd_plane_par(c, &q)) return BDGD_ERR_UNSUPPORTED;
   if (q.mode == PL_CPLX) return planes_launch_rt<T, PL_CPLX>(c, p, fd, q, x, ldx, y, ldy, spec, nc);
   if (q.mode == PL_WHOLE) return planes_launch_rt<T, PL_WHOLE>(c, p, fd, q, x, ldx, y, ldy, spec, nc);
+  // Compiled-in against run-time sizes, FP64 (FP32), us: Lrep of 16 columns 16^3
+  // 16 : 22 (12 : 19), 32^3 32 : 47 (24 : 35); 24 columns 48^3 115 : 151 (76 : 97);
+  // 32 columns 64^3 315 : 385 (207 : 267), 96^3 1215 : 1338 (686 : 953); 64
+  // columns 128^3 5562 : 6801 (2785 : 3707).  One column: 1.05 to 1.6 times.
   if (q.nx == q.ny && q.ny == q.nz) {
     switch (q.nx) {
 #define PLANE_CUBE(N) \
