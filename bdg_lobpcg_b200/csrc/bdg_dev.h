@@ -69,8 +69,6 @@ struct bdgd_ctx {
   size_t spec_bytes;
   void *io;   // staging for host applies
   size_t io_bytes;
-  void *pin;  // pinned host buffer of small host applies
-  size_t pin_bytes;
   double *gram_part;
   size_t gram_part_bytes;
   void *oz_buf;        // tensor-core Gram: column maxima of its operands + error flag (stream-ordered)

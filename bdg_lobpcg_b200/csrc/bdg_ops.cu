@@ -27,6 +27,7 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <mutex>
 #include <math.h>
 #include <stdarg.h>
 #include <stdio.h>
@@ -836,7 +837,6 @@ extern "C" void bdgd_destroy(bdgd_ctx **pc) {
     if (b) cudaFreeAsync(b, c->stream);
   if (c->stream) cudaStreamSynchronize(c->stream);
   if (c->stream) cudaStreamDestroy(c->stream);
-  if (c->pin) cudaFreeHost(c->pin);
   free(c);
   *pc = nullptr;
 }
@@ -1266,6 +1266,99 @@ static void graphs_clear(bdgd_ctx *c) {
   c->ngraphs = 0;
 }
 
+// Pinned staging buffers of small host applies, shared by all contexts and
+// threads; a call borrows one while it runs.  The driver's own staging of pageable
+// copies is slower, above all into pages that the caller has not touched yet: a
+// repeated Lrep of one 32^3 column takes 295 us without a buffer and 240 with one,
+// of 64^3 1.65 and 1.38 ms.  But page locking 0.5 MB takes 1.5 ms and 4 MB 5 ms, more
+// on a busy host: with a buffer in each context the first call of a new 32^3 context
+// took 1.9 ms against 1.05 without.  So a buffer of a size (a power of two) is made
+// when kPinCalls calls, about what it takes to earn it, have missed it.  At most
+// kPinSlots of kPinMax bytes; bdgd_trim gives back those not in use.
+static const size_t kPinMin = (size_t)64 << 10, kPinMax = (size_t)8 << 20;
+static const int kPinSlots = 4, kPinCalls = 32;
+static struct {
+  std::mutex mu;
+  struct {
+    void *p;
+    size_t bytes;
+    bool busy;
+  } slot[kPinSlots];
+  int missed[8];  // by size: kPinMin << i
+} g_pin;
+
+// a buffer of at least nb bytes, or -1
+static int pin_borrow(size_t nb) {
+  if (nb > kPinMax) return -1;
+  int cls = 0;
+  while ((kPinMin << cls) < nb) ++cls;
+  int i = -1;
+  void *old = nullptr;
+  {
+    std::lock_guard<std::mutex> l(g_pin.mu);
+    for (int q = 0; q < kPinSlots; ++q) {
+      const auto &s = g_pin.slot[q];
+      if (!s.busy && s.bytes >= nb && (i < 0 || s.bytes < g_pin.slot[i].bytes)) i = q;
+    }
+    if (i >= 0) {
+      g_pin.slot[i].busy = true;
+      return i;
+    }
+    if (++g_pin.missed[cls] < kPinCalls) return -1;
+    g_pin.missed[cls] = 0;
+    // in place of the smallest (an empty one has no bytes)
+    for (int q = 0; q < kPinSlots; ++q)
+      if (!g_pin.slot[q].busy && (i < 0 || g_pin.slot[q].bytes < g_pin.slot[i].bytes)) i = q;
+    if (i < 0) return -1;
+    auto &s = g_pin.slot[i];
+    s.busy = true;
+    old = s.p;
+    s.p = nullptr;
+    s.bytes = 0;
+  }
+  if (old) cudaFreeHost(old);
+  void *p = nullptr;
+  const bool ok = cudaMallocHost(&p, kPinMin << cls) == cudaSuccess;
+  if (!ok) cudaGetLastError();
+  std::lock_guard<std::mutex> l(g_pin.mu);
+  auto &s = g_pin.slot[i];
+  s.p = ok ? p : nullptr;
+  s.bytes = ok ? kPinMin << cls : 0;
+  s.busy = ok;
+  return ok ? i : -1;
+}
+
+static void pin_trim() {
+  for (int i = 0; i < kPinSlots; ++i) {
+    void *p = nullptr;
+    {
+      std::lock_guard<std::mutex> l(g_pin.mu);
+      auto &s = g_pin.slot[i];
+      if (s.busy) continue;
+      p = s.p;
+      s.p = nullptr;
+      s.bytes = 0;
+    }
+    if (p) cudaFreeHost(p);
+  }
+}
+
+// a borrowed buffer, returned when the copies queued with it are done
+struct PinLease {
+  const int i;
+  const cudaStream_t st;
+  PinLease(size_t nb, cudaStream_t s) : i(pin_borrow(nb)), st(s) {}
+  ~PinLease() {
+    if (i < 0) return;
+    cudaStreamSynchronize(st);
+    std::lock_guard<std::mutex> l(g_pin.mu);
+    g_pin.slot[i].busy = false;
+  }
+  PinLease(const PinLease &) = delete;
+  PinLease &operator=(const PinLease &) = delete;
+  void *get() const { return i < 0 ? nullptr : g_pin.slot[i].p; }
+};
+
 extern "C" int bdgd_trim(bdgd_ctx *c) {
   if (!c) return BDGD_ERR_ARG;
   BDGD_CK(cudaStreamSynchronize(c->stream));
@@ -1277,9 +1370,7 @@ extern "C" int bdgd_trim(bdgd_ctx *c) {
     *bufs[i] = nullptr;
     *sizes[i] = 0;
   }
-  if (c->pin) cudaFreeHost(c->pin);
-  c->pin = nullptr;
-  c->pin_bytes = 0;
+  pin_trim();
   c->version++;
   return BDGD_OK;
 }
@@ -1477,8 +1568,6 @@ extern "C" int bdgd_apply(bdgd_ctx *c, int op, int prec, const void *d_x, uint64
   return apply_tuned(c, op, p, prec, d_x, (long long)ldx, d_y, (long long)ldy, (int)ncol);
 }
 
-static const size_t kPinMax = (size_t)8 << 20;
-
 extern "C" int bdgd_apply_host(bdgd_ctx *c, int op, const void *x, void *y, uint64_t ncol) {
   const int two = (op == BDGD_OP_LREP || op == BDGD_OP_TLREP || op == BDGD_OP_SWAP) ? 2 : 1;
   const size_t esz = c->cplx ? 16 : 8;
@@ -1487,25 +1576,16 @@ extern "C" int bdgd_apply_host(bdgd_ctx *c, int op, const void *x, void *y, uint
   if (rc) return rc;
   char *dx = (char *)c->io;
   char *dy = dx + colb * ncol;
-  // Small columns go through a pinned buffer of the context: the driver's own
-  // staging of pageable copies is slower, above all into pages that the caller has
-  // not touched yet (Lrep of one 32^3 column: 267 -> 225 us a call).
   const size_t nb = colb * ncol;
-  if (nb <= kPinMax && c->pin_bytes < nb) {
-    if (c->pin) cudaFreeHost(c->pin);
-    c->pin = nullptr;
-    c->pin_bytes = 0;
-    if (cudaMallocHost(&c->pin, nb) == cudaSuccess) c->pin_bytes = nb;
-    else cudaGetLastError();
-  }
-  const bool pinned = nb <= kPinMax && c->pin_bytes >= nb;
-  if (pinned) memcpy(c->pin, x, nb);
-  BDGD_CK(cudaMemcpyAsync(dx, pinned ? c->pin : x, nb, cudaMemcpyHostToDevice, c->stream));
+  const PinLease lease(nb, c->stream);
+  void *pin = lease.get();
+  if (pin) memcpy(pin, x, nb);
+  BDGD_CK(cudaMemcpyAsync(dx, pin ? pin : x, nb, cudaMemcpyHostToDevice, c->stream));
   rc = bdgd_apply(c, op, BDGD_F64, dx, (uint64_t)c->S * two, dy, (uint64_t)c->S * two, ncol);
   if (rc) return rc;
-  BDGD_CK(cudaMemcpyAsync(pinned ? c->pin : y, dy, nb, cudaMemcpyDeviceToHost, c->stream));
+  BDGD_CK(cudaMemcpyAsync(pin ? pin : y, dy, nb, cudaMemcpyDeviceToHost, c->stream));
   BDGD_CK(cudaStreamSynchronize(c->stream));
-  if (pinned) memcpy(y, c->pin, nb);
+  if (pin) memcpy(y, pin, nb);
   return BDGD_OK;
 }
 

@@ -90,7 +90,8 @@ int bdgd_apply(bdgd_ctx *ctx, int op, int prec, const void *d_x, uint64_t ldx,
 int bdgd_set_graphs(bdgd_ctx *ctx, int on);
 
 /* Free the context's apply scratch (spectra, staging, Gram partials) and its
- * recorded graphs; they are reallocated on the next use. */
+ * recorded graphs, and the process's pinned staging buffers that no host apply
+ * is using; they are reallocated on the next use. */
 int bdgd_trim(bdgd_ctx *ctx);
 
 /* FFT pass family the autotuner chose for (op, prec) on this context: 0 not

@@ -6,11 +6,15 @@
   one chunk;
 * the FP32 plane kernels that prefetch (large applies) give the bits of
   one-column applies, which do not;
-* host applies below, at and above the size of the pinned staging buffer, growing
-  and shrinking, give the bits of device applies.
+* host applies below, at and above the largest pinned staging buffer, growing
+  and shrinking, before and after such buffers are made (32 calls of a size), and
+  from several threads at once, more than there are buffers, give the bits of
+  device applies.
 
 Tolerance against the generic kernels: 1e-12 of the largest entry (FP64).
 """
+import threading
+
 import numpy as np
 import pytest
 
@@ -97,21 +101,51 @@ def test_large_f32_applies_equal_single_columns(case, bdg, monkeypatch):
 
 
 @pytest.mark.parametrize("cplx", [False, True], ids=["d", "z"])
-def test_host_applies_around_the_pinned_buffer(cplx, bdg, monkeypatch):
+def test_host_applies_around_the_pinned_buffers(cplx, bdg, monkeypatch):
     torch = pytest.importorskip("torch")
     monkeypatch.setenv("BDG_FFT_PATH", "reg")
     N = [32, 32, 32]
     dc, S = _problem(bdg, N, cplx, 2)
     n = 2 * S
     col = n * (16 if cplx else 8)
-    full = (8 << 20) // col  # columns that fill the buffer
+    full = (8 << 20) // col  # columns that fill the largest buffer
     rng = np.random.default_rng(1)
-    for ncol in (1, full, full + 1, 2, 3 * full, full - 1, 1):
-        X = rng.standard_normal((ncol, n)) + (1j * rng.standard_normal((ncol, n)) if cplx else 0.0)
-        got = dc.apply_host(bdg.OP_LREP, X)
-        want = _apply(torch, dc, bdg.OP_LREP, 0, torch.tensor(X).cuda(), n)
-        assert np.array_equal(got, want.cpu().numpy()), ncol
-    # a context's scratch given back in between
+    for repeat in (1, 36):
+        for ncol in (1, full, full + 1, 2, 3 * full, full - 1, 1):
+            X = rng.standard_normal((ncol, n)) + (1j * rng.standard_normal((ncol, n)) if cplx else 0.0)
+            want = _apply(torch, dc, bdg.OP_LREP, 0, torch.tensor(X).cuda(), n).cpu().numpy()
+            for _ in range(repeat):
+                assert np.array_equal(dc.apply_host(bdg.OP_LREP, X), want), ncol
+    # buffers given back in between
     bdg.lib().bdgd_trim(dc.ptr)
-    assert np.array_equal(dc.apply_host(bdg.OP_LREP, X), got)
+    for _ in range(36):
+        assert np.array_equal(dc.apply_host(bdg.OP_LREP, X), want)
     dc.close()
+
+
+def test_host_applies_from_threads(bdg, monkeypatch):
+    torch = pytest.importorskip("torch")
+    monkeypatch.setenv("BDG_FFT_PATH", "reg")
+    rng = np.random.default_rng(4)
+    jobs = []
+    for i in range(7):
+        dc, S = _problem(bdg, [16, 16, 16 if i % 2 else 32], False, 20 + i)
+        X = rng.standard_normal((1 + i, 2 * S))
+        jobs.append((dc, X, _apply(torch, dc, bdg.OP_LREP, 0, torch.tensor(X).cuda(), 2 * S).cpu().numpy()))
+    bad = []
+
+    def work(dc, X, want, trim):
+        for k in range(80):
+            if not np.array_equal(dc.apply_host(bdg.OP_LREP, X), want):
+                bad.append(k)
+            if trim and k % 20 == 19:
+                bdg.lib().bdgd_trim(dc.ptr)
+
+    threads = [threading.Thread(target=work, args=j + (i == 3,)) for i, j in enumerate(jobs)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
+    for dc, _, _ in jobs:
+        dc.close()
