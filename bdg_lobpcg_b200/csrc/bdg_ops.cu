@@ -1057,6 +1057,20 @@ static int fft_path(const bdgd_ctx *c) {
   return FFT_PATH_REG;
 }
 
+// columns whose spectra the scratch cap admits at once
+static int spec_chunk(const bdgd_ctx *c, size_t per_col, int ncol) {
+  if (per_col * (size_t)ncol <= c->spec_cap) return ncol;
+  const int chunk = (int)(c->spec_cap / per_col);
+  return chunk < 1 ? 1 : chunk;
+}
+
+static int ensure_spec(bdgd_ctx *c, size_t bytes) {
+  void *before = c->spec;
+  const int rc = bdgd_ensure(c->stream, &c->spec, &c->spec_bytes, bytes);
+  if (!rc && c->spec != before) c->version++;  // captured graphs hold the old scratch
+  return rc;
+}
+
 template <typename T, bool CPLX>
 static int run_program(bdgd_ctx *c, const Prog &p, const void *x, long long ldx, void *y, long long ldy,
                        int ncol, int only_fwd, int only_bwd) {
@@ -1097,16 +1111,10 @@ static int run_program(bdgd_ctx *c, const Prog &p, const void *x, long long ldx,
   const bool planes = !only_fwd && !only_bwd && (path == FFT_PATH_REG || path == FFT_PATH_AUTO) &&
                       bdgd_planes_usable(c, prec) &&
                       !(path == FFT_PATH_AUTO && ncol < kTuneCols && lines && !bdgd_planes_pay(c, p, prec, ncol));
-  int chunk = ncol;
-  if (per_col * (size_t)chunk > c->spec_cap) {
-    chunk = (int)(c->spec_cap / per_col);
-    if (chunk < 1) chunk = 1;
-  }
-  if (only_fwd || only_bwd) chunk = ncol;  // raw transforms use the whole scratch as I/O
-  void *spec_before = c->spec;
-  int rc = bdgd_ensure(c->stream, &c->spec, &c->spec_bytes, per_col * (size_t)chunk);
+  // raw transforms use the whole scratch as I/O
+  const int chunk = only_fwd || only_bwd ? ncol : spec_chunk(c, per_col, ncol);
+  int rc = ensure_spec(c, per_col * (size_t)chunk);
   if (rc) return rc;
-  if (c->spec != spec_before) c->version++;  // captured graphs hold the old scratch
   C *spec = (C *)c->spec;
   const int tx = f32 ? 16 : 8;
   if (planes) {
@@ -1462,13 +1470,20 @@ static int apply_graph(bdgd_ctx *c, int op, const Prog &p, int prec, const void 
   return BDGD_OK;
 }
 
-// Choose the FFT pass family of (op, prec) on this context by timing each
-// (run twice, the second timed) on its first apply of >= 4 columns; later
-// applies use the fastest.  The register family has two forms, plane passes and
-// line passes: planes win by 1.1 to 1.7 on most grids, lines by up to 1.2 where
-// z is 256 long or one FP32 complex plane fills an SM (128^3 c64: 1077 against
-// 936 us for 8 columns), so both are timed where both can run.  BDG_FFT_PATH /
-// BDG_GENERIC_FFT override.
+// Choose the FFT pass family of (op, prec) on this context by timing each on its
+// first apply of >= kTuneCols columns; later applies use the fastest.  The register
+// family has two forms, plane passes and line passes: planes win by 1.1 to 1.7 on
+// most grids, lines by up to 1.2 where z is 256 long or one FP32 complex plane
+// fills an SM (128^3 c64: 1077 against 936 us for 8 columns), so both are timed
+// where both can run.  BDG_FFT_PATH / BDG_GENERIC_FFT override.
+//
+// What the first apply costs more than the others is kept below what it cost with
+// two families, each run twice: with three, one column warms lines and stages up
+// (loads their kernels; the plane kernels depend on the number of columns), and a
+// large block is timed on its first nt columns, still thousands of thread blocks a
+// launch, then applied.  First apply, us (two families before, three now):
+// Lrep FP64 48^3 x 24 1360 -> 1060, 64^3 x 32 2960 -> 2260, 128^3 x 64 45000 -> 8410;
+// with every family run twice on the part it was 1610, 3620 and 15100.
 static int apply_tuned(bdgd_ctx *c, int op, const Prog &p, int prec, const void *x, long long ldx, void *y,
                        long long ldy, int ncol) {
   const int pi = prec == BDGD_F32 ? 1 : 0;
@@ -1479,36 +1494,30 @@ static int apply_tuned(bdgd_ctx *c, int op, const Prog &p, int prec, const void 
     float ms[4] = {0.f, 0.f, 0.f, 0.f};
     const bool planes = bdgd_planes_usable(c, prec);
     const int order[3] = {2, planes ? 3 : 1, 1};  // the likely choice last: its result stays in y
-    // A block of many columns is timed on its first nt, still thousands of thread
-    // blocks a launch, between two applies of the whole (the first sizes the
-    // scratch, the second is the result): two whole applies and six partial ones
-    // in place of six whole ones.
     const long long fill = ((1LL << 23) + c->S - 1) / c->S;
     const int nt = (int)(fill < 4 ? 4 : fill) < ncol ? (int)(fill < 4 ? 4 : fill) : ncol;
-    cudaEvent_t e0, e1;
-    BDGD_CK(cudaEventCreate(&e0));
-    BDGD_CK(cudaEventCreate(&e1));
-    int rc = BDGD_OK;
-    if (nt < ncol) {
-      c->force_path = 1;
-      rc = dispatch(c, p, prec, x, ldx, y, ldy, ncol, 0, 0);
-    }
-    for (int i = 0; i < (planes ? 3 : 2) && !rc; ++i) {
+    cudaEvent_t e[3][2] = {};
+    const auto ck = [](cudaError_t ce) { return ce == cudaSuccess ? BDGD_OK : bdgd_check(ce, "autotune"); };
+    const int nfam = planes ? 3 : 2;
+    // the whole block's scratch first: no reallocation between the runs
+    const size_t per_col = (size_t)p.J * c->geo.H * (prec == BDGD_F32 ? sizeof(float2) : sizeof(double2));
+    int rc = ensure_spec(c, per_col * (size_t)spec_chunk(c, per_col, ncol));
+    for (int i = 0; i < nfam && !rc; ++i) {
+      for (int q = 0; q < 2 && !rc; ++q) rc = ck(cudaEventCreate(&e[i][q]));
       const int k = order[i];
       c->force_path = k;
-      rc = dispatch(c, p, prec, x, ldx, y, ldy, nt, 0, 0);
-      if (!rc) {
-        cudaEventRecord(e0, c->stream);
-        rc = dispatch(c, p, prec, x, ldx, y, ldy, nt, 0, 0);
-        cudaEventRecord(e1, c->stream);
-        cudaError_t ce = cudaEventSynchronize(e1);
-        if (ce != cudaSuccess) rc = bdgd_check(ce, "autotune");
-        else cudaEventElapsedTime(&ms[k], e0, e1);
-      }
+      if (!rc) rc = dispatch(c, p, prec, x, ldx, y, ldy, planes && k != 1 ? 1 : nt, 0, 0);
+      if (!rc) cudaEventRecord(e[i][0], c->stream);
+      if (!rc) rc = dispatch(c, p, prec, x, ldx, y, ldy, nt, 0, 0);
+      if (!rc) cudaEventRecord(e[i][1], c->stream);
+    }
+    if (!rc) rc = ck(cudaEventSynchronize(e[nfam - 1][1]));
+    for (int i = 0; i < nfam; ++i) {
+      if (!rc) cudaEventElapsedTime(&ms[order[i]], e[i][0], e[i][1]);
+      for (int q = 0; q < 2; ++q)
+        if (e[i][q]) cudaEventDestroy(e[i][q]);
     }
     c->force_path = 0;
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
     if (rc) return rc;
     c->tune_lines[op][pi] = planes && ms[3] < ms[1];
     const float reg = c->tune_lines[op][pi] ? ms[3] : ms[1];
