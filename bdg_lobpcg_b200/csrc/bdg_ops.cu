@@ -863,11 +863,12 @@ __global__ void k_ptab(GeoDev g, FieldsDev f, double *__restrict__ out) {
   }
 }
 
-// End of a setter: the caller may change its arrays.  A host apply waits once, at
-// its end, for the uploads before it too.
-static int upload_done(bdgd_ctx *c) {
-  if (!c->host_apply) BDGD_CK(cudaStreamSynchronize(c->stream));
-  return BDGD_OK;
+// End of a setter, with its error if one upload failed: the caller may change its
+// arrays.  A host apply waits once, at its end, for the uploads before it too.
+static int upload_done(bdgd_ctx *c, int rc = BDGD_OK) {
+  if (!c->host_apply && rc) cudaStreamSynchronize(c->stream);
+  else if (!c->host_apply) BDGD_CK(cudaStreamSynchronize(c->stream));
+  return rc;
 }
 
 static int build_ptab(bdgd_ctx *c) {
@@ -899,16 +900,16 @@ extern "C" void bdgd_host_apply(bdgd_ctx *c, int on) { c->host_apply = on; }
 extern "C" int bdgd_set_local_terms(bdgd_ctx *c, const double *ltK, const double *ltM) {
   c->version++;
   int rc;
-  if (ltK && (rc = upload_pair(c, &c->ltK64, &c->ltK32, ltK, c->S))) return rc;
-  if (ltM && (rc = upload_pair(c, &c->ltM64, &c->ltM32, ltM, c->S))) return rc;
+  if (ltK && (rc = upload_pair(c, &c->ltK64, &c->ltK32, ltK, c->S))) return upload_done(c, rc);
+  if (ltM && (rc = upload_pair(c, &c->ltM64, &c->ltM32, ltM, c->S))) return upload_done(c, rc);
   return upload_done(c);
 }
 
 extern "C" int bdgd_set_precond(bdgd_ctx *c, const double *sK, const double *sM, double mu) {
   c->version++;
   int rc;
-  if (sK && (rc = upload_pair(c, &c->pK64, &c->pK32, sK, c->S))) return rc;
-  if (sM && (rc = upload_pair(c, &c->pM64, &c->pM32, sM, c->S))) return rc;
+  if (sK && (rc = upload_pair(c, &c->pK64, &c->pK32, sK, c->S))) return upload_done(c, rc);
+  if (sM && (rc = upload_pair(c, &c->pM64, &c->pM32, sM, c->S))) return upload_done(c, rc);
   c->mu = mu;
   c->has_precond = (sK && sM) ? 1 : c->has_precond;
   return build_ptab(c);
@@ -923,7 +924,7 @@ extern "C" int bdgd_set_wavefunction(bdgd_ctx *c, const void *wf) {
   int rc = upload_pair(c, &d64, &d32, (const double *)wf, n);
   c->wf64 = d64;
   c->wf32 = d32;
-  if (rc) return rc;
+  if (rc) return upload_done(c, rc);
   c->has_wf = 1;
   return upload_done(c);
 }
